@@ -151,6 +151,39 @@ int upload_tables(gt_handle* h, DevTables<R>& t) {
   };
   const size_t o_twx = puttw(g.nx), o_twy = puttw(g.ny), o_twz = puttw(g.nz);
   const size_t o_twzh = puttw(g.nz >= 2 ? g.nz / 2 : 1);
+  // The same tables as fixed-point limbs (FP64 form): cos and sin in Q62,
+  // rounded to nearest, as c1 2^32 + c0 with signed limbs (c0 kept off
+  // -2^31, whose negative has no int).  Only the per-stage entries are read.
+  auto limbs = [](long double v, int32_t* o) {
+    int64_t q = llrintl(v * 4611686018427387904.0L);
+    if ((int32_t)q == INT32_MIN) ++q;
+    o[1] = (int32_t)q;
+    o[0] = (int32_t)((q - o[1]) >> 32);
+  };
+  auto putfw = [&](int L) {
+    std::vector<int32_t> c(8 * (size_t)L, 0);
+    const int lgl = ilog2(L);
+    size_t off = 0;
+    for (int lgns = 0; lgns < lgl;) {
+      const int lr = lgl - lgns >= 3 ? 3 : lgl - lgns;
+      const int r = 1 << lr, ns = 1 << lgns;
+      if (lgns > 0) {
+        for (int j = 1; j < r; ++j)
+          for (int k = 0; k < ns; ++k) {
+            long double cv, sv;
+            cos_sin((int)((size_t)j * k * (L / (ns * r))), L, cv, sv);
+            int32_t* e = &c[4 * (L + off + (size_t)(j - 1) * ns + k)];
+            limbs(cv, e);
+            limbs(-sv, e + 2);
+          }
+        off += (size_t)(r - 1) * ns;
+      }
+      lgns += lr;
+    }
+    return put(c.data(), c.size() * sizeof(int32_t));
+  };
+  const bool fx = sizeof(R) == 8;
+  const size_t o_fwx = fx ? putfw(g.nx) : 0, o_fwy = fx ? putfw(g.ny) : 0, o_fwz = fx ? putfw(g.nz) : 0;
   std::vector<int32_t> tiles;
   build_ztiles(g, ht.xcut.data(), (int)sizeof(Cplx<R>), tiles);
   if (tiles.empty()) tiles = {0, 0};
@@ -192,6 +225,9 @@ int upload_tables(gt_handle* h, DevTables<R>& t) {
   t.twy = dptr<const void>(mem, o_twy);
   t.twz = dptr<const void>(mem, o_twz);
   t.twzh = dptr<const void>(mem, o_twzh);
+  t.fwx = fx ? dptr<const void>(mem, o_fwx) : nullptr;
+  t.fwy = fx ? dptr<const void>(mem, o_fwy) : nullptr;
+  t.fwz = fx ? dptr<const void>(mem, o_fwz) : nullptr;
   t.omega = (R)h->p.omega;
   t.dt = (R)h->p.dt;
   t.dt2 = (R)(h->p.dt2_mode == GT_DT2_RK2 ? 0.5 * h->p.dt : 0.0);
@@ -509,6 +545,9 @@ int gtc::create_handle(const gt_params* p, gt_handle** out, void* ext_fields) {
   }
   for (int c = 0; c < 6; ++c) h->w[c] = dptr<void>(h->fields_mem, (6 + c) * fbytes);
   CKH(cudaMalloc(&h->stage, g.field_elems() * 16));
+  // the FP64 passes' line exponents live in the staging field, which only
+  // transfers use otherwise (in stream order with the passes)
+  if (!h->mixed) h->pm.fx_scratch = h->stage;
   rc = h->mixed ? upload_tables<float>(h, h->t32) : upload_tables<double>(h, h->t64);
   if (rc) { free_handle(h); return rc; }
   const int nbin = g.nx / 2;

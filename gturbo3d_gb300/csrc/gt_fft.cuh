@@ -18,12 +18,25 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 namespace gt {
 
+// A transform's values are float2, or longlong2 in block fixed point (the
+// FP64 form, gt_fixed.cuh); double2 is the FP64 form's storage.
+using i64 = long long;
 template <typename R> struct CplxOf;
 template <> struct CplxOf<float> { using type = float2; };
 template <> struct CplxOf<double> { using type = double2; };
+template <> struct CplxOf<i64> { using type = longlong2; };
 template <typename R> using Cplx = typename CplxOf<R>::type;
+
+// A table twiddle e^{-2 pi i m / L}: a complex value, or for fixed-point
+// transforms cos and sin in Q62 as balanced 32-bit limbs {c1, c0, s1, s0}
+// (value c1 2^32 + c0, both signed).
+template <typename R> struct TwOf { using type = Cplx<R>; };
+template <> struct TwOf<i64> { using type = int4; };
+template <typename R> using Tw = typename TwOf<R>::type;
 
 template <typename C> __device__ __forceinline__ C cadd(C a, C b) { return C{a.x + b.x, a.y + b.y}; }
 template <typename C> __device__ __forceinline__ C csub(C a, C b) { return C{a.x - b.x, a.y - b.y}; }
@@ -103,6 +116,52 @@ template <int SIGN, typename R> __device__ __forceinline__ CTrip<R> twmul(CTrip<
   return CTrip<R>{twmul<SIGN>(p.a, w), twmul<SIGN>(p.b, w), twmul<SIGN>(p.c, w)};
 }
 
+// ---- 64-bit fixed point (longlong2) ---------------------------------------
+// a * b + c, 32 x 32 -> 64 bits: one instruction of the integer multiply pipe.
+__device__ __forceinline__ i64 mad_wide(int a, int b, i64 c) {
+  i64 r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
+// x = x1 2^32 + x0 with both limbs signed.
+struct Limbs {
+  int x1, x0;
+  __device__ __forceinline__ explicit Limbs(i64 x) {
+    x0 = (int)x;
+    x1 = (int)(x >> 32) + (int)((unsigned)x0 >> 31);
+  }
+};
+// a * w or a * conj(w) for a Q62 twiddle, times 2^-f (f <= 2; rnd = 2^(29 + f)):
+// the limb products but the lowest (below one unit), the middle ones summed at
+// full width and rounded.  |a| < 2^61 keeps the sums inside 64 bits and 4 a1
+// inside 32.
+template <int SIGN> __device__ __forceinline__ longlong2 twmul(longlong2 a, int4 w, int f = 0, i64 rnd = 1ll << 29) {
+  const Limbs r(a.x), i(a.y);
+  const int s1 = SIGN < 0 ? w.z : -w.z, s0 = SIGN < 0 ? w.w : -w.w;   // im of the factor
+  const int n1 = -s1, n0 = -s0;
+  i64 mr = mad_wide(r.x1, w.y, rnd), mi = mad_wide(r.x1, s0, rnd);
+  mr = mad_wide(r.x0, w.x, mr);
+  mi = mad_wide(r.x0, s1, mi);
+  mr = mad_wide(i.x1, n0, mr);
+  mi = mad_wide(i.x1, w.y, mi);
+  mr = mad_wide(i.x0, n1, mr);
+  mi = mad_wide(i.x0, w.x, mi);
+  const int r4 = r.x1 << (2 - f), i4 = i.x1 << (2 - f);
+  longlong2 o;
+  o.x = mad_wide(i4, n1, mad_wide(r4, w.x, mr >> (30 + f)));
+  o.y = mad_wide(i4, w.x, mad_wide(r4, s1, mi >> (30 + f)));
+  return o;
+}
+// sqrt(1/2) x, rounded, |x| < 2^62: the constant in Q63 as c1 2^32 + c0, the
+// low limb of x unsigned (c1 > 0; the dropped product is below 0.05 units).
+__device__ __forceinline__ i64 sqrt_half(i64 x) {
+  constexpr int c1 = 1518500250, c0 = -51432894;
+  const int x1 = (int)(x >> 32);
+  i64 m = mad_wide(x1, c0, 1ll << 30);
+  asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(m) : "r"((unsigned)x), "r"((unsigned)c1));
+  return mad_wide(x1 << 1, c1, m >> 31);
+}
+
 template <typename C> __device__ __forceinline__ void dft2(C& a, C& b) {
   const C t = a;
   a = cadd(t, b);
@@ -122,12 +181,22 @@ template <int SIGN, typename C> __device__ __forceinline__ void dft4(C& x0, C& x
 // forward), and the radix-2 combination e +- o of such a product written
 // component-wise so that the products fuse into FMAs.
 template <int SIGN, typename R> __device__ __forceinline__ Cplx<R> w8_1(Cplx<R> o) {
-  const R c = (R)0.70710678118654752440;
-  return SIGN < 0 ? Cplx<R>{c * (o.x + o.y), c * (o.y - o.x)} : Cplx<R>{c * (o.x - o.y), c * (o.x + o.y)};
+  if constexpr (std::is_same_v<R, i64>) {
+    return SIGN < 0 ? Cplx<R>{sqrt_half(o.x + o.y), sqrt_half(o.y - o.x)}
+                    : Cplx<R>{sqrt_half(o.x - o.y), sqrt_half(o.x + o.y)};
+  } else {
+    const R c = (R)0.70710678118654752440;
+    return SIGN < 0 ? Cplx<R>{c * (o.x + o.y), c * (o.y - o.x)} : Cplx<R>{c * (o.x - o.y), c * (o.x + o.y)};
+  }
 }
 template <int SIGN, typename R> __device__ __forceinline__ Cplx<R> w8_3(Cplx<R> o) {
-  const R c = (R)0.70710678118654752440;
-  return SIGN < 0 ? Cplx<R>{c * (o.y - o.x), -c * (o.x + o.y)} : Cplx<R>{-c * (o.x + o.y), c * (o.x - o.y)};
+  if constexpr (std::is_same_v<R, i64>) {
+    return SIGN < 0 ? Cplx<R>{sqrt_half(o.y - o.x), -sqrt_half(o.x + o.y)}
+                    : Cplx<R>{-sqrt_half(o.x + o.y), sqrt_half(o.x - o.y)};
+  } else {
+    const R c = (R)0.70710678118654752440;
+    return SIGN < 0 ? Cplx<R>{c * (o.y - o.x), -c * (o.x + o.y)} : Cplx<R>{-c * (o.x + o.y), c * (o.x - o.y)};
+  }
 }
 template <typename C> __device__ __forceinline__ C fadd(C e, C o) { return C{e.x + o.x, e.y + o.y}; }
 template <typename C> __device__ __forceinline__ C fsub(C e, C o) { return C{e.x - o.x, e.y - o.y}; }
@@ -202,10 +271,10 @@ template <typename R, int LGL, int LGNS> struct StageTw {
   static constexpr int NS = 1 << LGNS;
   static constexpr int T = 1 << (LGL - 3);
   static constexpr int N = LGNS == 0 ? 1 : (LR == 3 ? 7 : (LR == 2 ? 6 : 4));
-  Cplx<R> w[N];
-  __device__ __forceinline__ void load(int t, const Cplx<R>* __restrict__ tw) {
+  Tw<R> w[N];
+  __device__ __forceinline__ void load(int t, const Tw<R>* __restrict__ tw) {
     if constexpr (LGNS > 0) {
-      const Cplx<R>* tws = tw + (1 << LGL) + tw_stage_offset(LGL, LGNS);
+      const Tw<R>* tws = tw + (1 << LGL) + tw_stage_offset(LGL, LGNS);
       if constexpr (LR == 3) {
         const int k = t & (NS - 1);
 #pragma unroll
@@ -255,7 +324,7 @@ template <typename R, typename Idx> struct TripMem {
 // PF: twiddles a stage ahead (FP32 default: measured faster); otherwise at
 // the stage itself (FP64: the extra live registers spill in the z pass).
 template <int SIGN, typename R, int LGL, int LGNS, bool PF, typename E, typename Mem, typename Sync>
-__device__ __forceinline__ void fft_stages_ct(E v[8], int t, const Cplx<R>* __restrict__ tw, const Mem& mem,
+__device__ __forceinline__ void fft_stages_ct(E v[8], int t, const Tw<R>* __restrict__ tw, const Mem& mem,
                                               const Sync& sync, const StageTw<R, LGL, LGNS>& cur) {
   constexpr int REM = LGL - LGNS;
   constexpr int LR = REM >= 3 ? 3 : REM;

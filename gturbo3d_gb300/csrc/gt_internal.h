@@ -85,6 +85,9 @@ struct DevTables {
   const void* twy;      // ny
   const void* twz;      // nz
   const void* twzh;     // nz / 2 (the half-length z transforms of the cluster-pair z passes)
+  const void* fwx;      // FP64 form: the same per-axis tables as fixed-point limbs (gt_fixed.cuh)
+  const void* fwy;
+  const void* fwz;
   R omega, dt, dt2, scale;  // scale = 1/(nx ny nz)
   int truncate;
   // Truncation-aware pruning (truncate = 1 and a state that is zero outside
@@ -148,6 +151,8 @@ struct PassTuning {
   int z_cluster = 0;        // FP32: 1 = the z forward pass on cluster pairs of CTAs, each holding half
                             // of a tile's z-rows (two tiles per SM; the default for z columns of 1024
                             // points or more); 0 = one CTA per tile
+  void* fx_scratch = nullptr;  // FP64: the fixed-point passes' line exponents (nullptr: FP64 arithmetic),
+  long long fx_stride = 0;     // members of a batched launch this many ints apart
   void* stream2 = nullptr;  // the handle's second stream and the events for overlap / slab_pipe
   void* ev_fork = nullptr;
   void* ev_join = nullptr;

@@ -2238,6 +2238,12 @@ k_final_sum(const double* __restrict__ partials, int nblocks, int nq, double* __
   }
 }
 
+#ifdef GT_KERNELS_FX
+}  // namespace gt
+#include "gt_fx_kernels.cuh"
+namespace gt {
+#endif
+
 // ---------------------------------------------------------------------------
 // Launch configuration.
 // ---------------------------------------------------------------------------
@@ -2311,7 +2317,7 @@ static int set_smem_attrs() {
   int optin = 0;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return (int)e;
-  cudaError_t es[8 * 24 + 1];
+  cudaError_t es[8 * 32 + 1];
   int n = 0;
 #define GT_ALLOW(LG)                                     \
   es[n++] = allow_smem(k_zinv_curl<R, LG>, optin);       \
@@ -2340,6 +2346,18 @@ static int set_smem_attrs() {
   es[n++] = allow_smem(k_xr2c<R, LG>, optin);
   GT_ALLOW(3) GT_ALLOW(4) GT_ALLOW(5) GT_ALLOW(6) GT_ALLOW(7) GT_ALLOW(8) GT_ALLOW(9) GT_ALLOW(10)
 #undef GT_ALLOW
+#ifdef GT_KERNELS_FX
+#define GT_ALLOW(LG)                              \
+  es[n++] = allow_smem(k_fx_zinv<LG>, optin);     \
+  es[n++] = allow_smem(k_fx_spass<0, LG>, optin); \
+  es[n++] = allow_smem(k_fx_spass<1, LG>, optin); \
+  es[n++] = allow_smem(k_fx_spass<2, LG>, optin); \
+  es[n++] = allow_smem(k_fx_spass<3, LG>, optin); \
+  es[n++] = allow_smem(k_fx_x<LG>, optin);        \
+  es[n++] = allow_smem(k_fx_zfwd<LG>, optin);
+  GT_ALLOW(3) GT_ALLOW(4) GT_ALLOW(5) GT_ALLOW(6) GT_ALLOW(7) GT_ALLOW(8) GT_ALLOW(9) GT_ALLOW(10)
+#undef GT_ALLOW
+#endif
   es[n++] = allow_smem(k_diag<R>, optin);
   for (int i = 0; i < n; ++i)
     if (es[i] != cudaSuccess) return (int)es[i];
@@ -2494,10 +2512,97 @@ static int spass(const Geom& g, void* const* fields, int nf, const void* tw, int
   return (int)cudaGetLastError();
 }
 
-template <typename R>
+#ifdef GT_KERNELS_FX
+// A strided pass in fixed point (KIND of k_fx_spass): z for KIND 2 and 3, else y.
+template <int KIND>
+static int fx_spass(const Geom& g, void* const* fields, int nf, const void* tw, cudaStream_t s, LaunchHook hook,
+                    void* hctx, const FxExp& ex, int xlim = -1, int ymask = 0, const int32_t* xcut0 = nullptr,
+                    int nmem = 1, long long fxs = 0, long long mstride = 0) {
+  constexpr bool zaxis = KIND >= 2;
+  const int lgL = zaxis ? g.lnz : g.lny;
+  const long long plane = (long long)g.ny * g.nhp;
+  const long long ls = zaxis ? plane : g.nhp, os = zaxis ? g.nhp : plane;
+  if (xlim < 0) xlim = g.nh;
+  const int TX = 1 << fx_lg_tile(lgL), smem = strided_rows(1 << lgL) * TX * 16;
+  Ptr6 f{};
+  for (int i = 0; i < nf; ++i) f.p[i] = fields[i];
+  const dim3 grid((xlim + TX - 1) / TX, zaxis ? g.ny : g.nz, nf * nmem);
+  const int kind = KIND == 0 || KIND == 2 ? kKYPass : kKYFwd;
+  GT_HOOK(kind, true);
+#define GT_L(LG)                                                                                              \
+  k_fx_spass<KIND, LG><<<grid, kFxTileThreads, smem, s>>>(f, g, tw, ls, os, xlim, ymask, xcut0, nf, ex, fxs, mstride);
+  GT_DISPATCH_LG(lgL, GT_L)
+#undef GT_L
+  GT_HOOK(kind, false);
+  return (int)cudaGetLastError();
+}
+
+// One nonlinear term of the FP64 form with its transforms in fixed point.  The
+// knobs that select another kernel for a pass keep FP64 arithmetic throughout
+// (nlt_phases), since the work fields' format is shared by the passes.
+static bool fx_applies(const PassTuning* pm, unsigned nm) {
+  return pm && pm->fx_scratch && (nm == 1 || pm->fx_stride > 0) && pm->x_fused == 2 && !pm->z_split &&
+         !pm->overlap && !pm->slab_pipe && !pm->zf_pipe && !pm->fuse_stage;
+}
+
+static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], void* const bcor[3],
+                  void* const out[3], void* const w[6], int mode, int pruned, const PassTuning* pm, cudaStream_t s,
+                  LaunchHook hook, void* hctx, const Batch<double>& bb) {
+  const unsigned nm = bb.nmem > 0 ? (unsigned)bb.nmem : 1u;
+  const long long mstride = bb.nmem > 0 ? bb.mstride : 0, fxs = nm > 1 ? pm->fx_stride : 0;
+  const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
+  int rc = (int)(nm > 1 ? cudaMemset2DAsync(ex.mz, (size_t)fxs * sizeof(int), kFxUnsetByte, ex.max_bytes, nm, s)
+                        : cudaMemsetAsync(ex.mz, kFxUnsetByte, ex.max_bytes, s));
+  if (rc) return rc;
+  const int lgt = fx_lg_tile(g.lnz), zsmem = strided_rows(g.nz) * (16 << lgt);
+  const dim3 zgrid = pruned ? dim3(tb.nztl[lgt], nm) : dim3((g.nh + (1 << lgt) - 1) >> lgt, g.ny, nm);
+  Ptr6 pa{}, pw{}, pb{}, po{};
+  for (int i = 0; i < 6; ++i) pw.p[i] = w[i];
+  for (int i = 0; i < 3; ++i) {
+    pa.p[i] = a[i];
+    pb.p[i] = bcor[i];
+    po.p[i] = out[i];
+  }
+  GT_HOOK(kKZinvCurl, true);
+#define GT_L(LG) \
+  k_fx_zinv<LG><<<zgrid, kFxTileThreads, zsmem, s>>>(pa, pw, tb, g, pruned, tb.ztl[lgt], ex, fxs, mstride);
+  GT_DISPATCH_LG(g.lnz, GT_L)
+#undef GT_L
+  GT_HOOK(kKZinvCurl, false);
+  if ((rc = (int)cudaGetLastError())) return rc;
+  const int xlim = pruned ? tb.xa : g.nh;
+  if ((rc = fx_spass<0>(g, w, 6, tb.fwy, s, hook, hctx, ex, xlim, pruned ? 1 : 0, tb.xcut, (int)nm, fxs, mstride)))
+    return rc;
+  {
+    // whole warps: 96 threads (32 / (nx / 8) pairs) up to nx = 256, one pair above; ny nz / 2 is a multiple
+    const long long npairs = (long long)g.ny * g.nz / 2;
+    const int P = g.nx >= 256 ? 1 : 256 / g.nx;
+    GT_HOOK(kKXCross, true);
+#define GT_L(LG)                                                                                        \
+  k_fx_x<LG><<<dim3((unsigned)(npairs / P), nm), fx_x_threads<LG>(), 3 * P * strided_rows(g.nx) * 16, s>>>(              \
+      pw, g, tb.fwx, xlim, g.lnx + g.lny + g.lnz, ex, fxs, mstride);
+    GT_DISPATCH_LG(g.lnx, GT_L)
+#undef GT_L
+    GT_HOOK(kKXCross, false);
+    if ((rc = (int)cudaGetLastError())) return rc;
+  }
+  if ((rc = fx_spass<1>(g, w, 3, tb.fwy, s, hook, hctx, ex, xlim, pruned ? 2 : 0, tb.xcut, (int)nm, fxs, mstride)))
+    return rc;
+  GT_HOOK(kKZFwdEpi, true);
+#define GT_L(LG)                                                                                                  \
+  k_fx_zfwd<LG><<<zgrid, kFxTileThreads, 3 * zsmem, s>>>(pw, pb, po, tb, g, mode, pruned, tb.ztl[lgt], ex, fxs, bb);
+  GT_DISPATCH_LG(g.lnz, GT_L)
+#undef GT_L
+  GT_HOOK(kKZFwdEpi, false);
+  return (int)cudaGetLastError();
+}
+
+#endif  // GT_KERNELS_FX
+
 // The passes of one nonlinear term; `phases` selects pass 1 (bit 0), passes
 // 2-4 (bit 1) and pass 5 (bit 2), so that the RK2 step can run the stage
 // boundary as one fused kernel in between.
+template <typename R>
 static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], void* const bcor[3],
                       void* const out[3], void* const w[6], int mode, int pruned, const PassTuning* pm,
                       int* err, void* stream, LaunchHook hook, void* hctx, int phases,
@@ -2509,6 +2614,10 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
   const unsigned nm = bb.nmem > 0 ? (unsigned)bb.nmem : 1u;
   const long long mstride = bb.nmem > 0 ? bb.mstride : 0;
   cudaStream_t s = (cudaStream_t)stream;
+#ifdef GT_KERNELS_FX
+  if (phases == 7 && fx_applies(pm, nm))
+    return fx_nlt(g, tb, a, bcor, out, w, mode, pruned, pm, s, hook, hctx, bb);
+#endif
   const int csize = sizeof(Cplx<R>);
   // z tiles: 16 columns (128-byte row segments, one block of three 512-row
   // fields per SM) for FP32 z columns of 256 points or more, where they
@@ -2909,8 +3018,24 @@ int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* spec, void* real
   int rc = set_smem_attrs<R>();
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  (void)w;
   void* f[1] = {spec};
+#ifdef GT_KERNELS_FX
+  // fixed point, the line exponents in w[2] (no caller keeps a field there)
+  const FxExp ex = fx_exp(w[2], g.ny, g.nz, g.nhp);
+  if ((rc = (int)cudaMemsetAsync(ex.mz, kFxUnsetByte, ex.max_bytes, s))) return rc;
+  if ((rc = fx_spass<2>(g, f, 1, tb.fwz, s, hook, hctx, ex))) return rc;
+  if ((rc = fx_spass<0>(g, f, 1, tb.fwy, s, hook, hctx, ex))) return rc;
+  const int P = xpass_pairs(g, 1, 16, 256, 1);
+  GT_HOOK(kKFft1, true);
+#define GT_L(LG)                                                                                  \
+k_fx_xc2r<LG><<<(unsigned)((long long)g.ny * g.nz / 2 / P), P * (g.nx / 8), P * strided_rows(g.nx) * 16, s>>>( \
+    spec, reinterpret_cast<double*>(real_out), g, tb.fwx, P, ex);
+  GT_DISPATCH_LG(g.lnx, GT_L)
+#undef GT_L
+  GT_HOOK(kKFft1, false);
+  return (int)cudaGetLastError();
+#else
+  (void)w;
   if ((rc = spass<R>(g, f, 1, tb.twz, 2, +1, s, hook, hctx))) return rc;
   if ((rc = spass<R>(g, f, 1, tb.twy, 1, +1, s, hook, hctx))) return rc;
   const int csize = sizeof(Cplx<R>);
@@ -2925,6 +3050,7 @@ int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* spec, void* real
 #undef GT_L
   GT_HOOK(kKFft1, false);
   return (int)cudaGetLastError();
+#endif
 }
 
 template <typename R>
@@ -2933,6 +3059,22 @@ int launch_fft_dir(const Geom& g, const DevTables<R>& tb, const void* real_in, v
   int rc = set_smem_attrs<R>();
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
+#ifdef GT_KERNELS_FX
+  const FxExp ex = fx_exp(w[2], g.ny, g.nz, g.nhp);   // as in launch_fft_inv
+  if ((rc = (int)cudaMemsetAsync(ex.mz, kFxUnsetByte, ex.max_bytes, s))) return rc;
+  const int P = xpass_pairs(g, 1, 16, 256, 1);
+  GT_HOOK(kKFft1, true);
+#define GT_L(LG)                                                                                  \
+k_fx_xr2c<LG><<<(unsigned)((long long)g.ny * g.nz / 2 / P), P * (g.nx / 8), P * strided_rows(g.nx) * 16, s>>>( \
+    reinterpret_cast<const double*>(real_in), spec_out, g, tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
+  GT_DISPATCH_LG(g.lnx, GT_L)
+#undef GT_L
+  GT_HOOK(kKFft1, false);
+  if ((rc = (int)cudaGetLastError())) return rc;
+  void* f[1] = {spec_out};
+  if ((rc = fx_spass<1>(g, f, 1, tb.fwy, s, hook, hctx, ex))) return rc;
+  return fx_spass<3>(g, f, 1, tb.fwz, s, hook, hctx, ex);
+#else
   (void)w;
   const int csize = sizeof(Cplx<R>);
   const int P = xpass_pairs(g, 1, csize, max_threads<R>(), 1);
@@ -2950,6 +3092,7 @@ int launch_fft_dir(const Geom& g, const DevTables<R>& tb, const void* real_in, v
   void* f[1] = {spec_out};
   if ((rc = spass<R>(g, f, 1, tb.twy, 1, -1, s, hook, hctx))) return rc;
   return spass<R>(g, f, 1, tb.twz, 2, -1, s, hook, hctx);
+#endif
 }
 
 template <typename R>
