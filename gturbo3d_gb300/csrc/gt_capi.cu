@@ -22,6 +22,8 @@ thread_local std::string g_last_error;
 
 }  // namespace
 
+size_t gtc::spec_bytes(const Geom& g) { return (size_t)g.nh * g.ny * g.nz * 16; }
+
 int gtc::cuda_fail(cudaError_t e, const char* what) {
   g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
   return GT_ECUDA;
@@ -341,52 +343,46 @@ int force(gt_handle* h, const ForceEntry* d, int n, int serial) {
   return launch_force<double>(h->g, h->b, d, n, serial, h->stream, hook_fn, h);
 }
 
-// FP64 staging [n complex] <-> working precision
-int to_working(gt_handle* h, const void* stage, void* dst, size_t n) {
+// FP64 staging <-> FP32, n complex values (mixed form).
+int convert_real(gt_handle* h, const void* src, void* dst, size_t n, int to_working) {
   Geom g1 = h->g;
   g1.nz = 1; g1.ny = 1; g1.nhp = (int)n;   // field_elems() == n
-  if (h->mixed) return launch_convert<float>(g1, stage, dst, 1, h->stream, hook_fn, h);
-  CK(cudaMemcpyAsync(dst, stage, n * 16, cudaMemcpyDeviceToDevice, h->stream));
-  return 0;
+  return launch_convert<float>(g1, src, dst, to_working, h->stream, hook_fn, h);
 }
 
-int from_working(gt_handle* h, const void* src, void* stage, size_t n) {
-  Geom g1 = h->g;
-  g1.nz = 1; g1.ny = 1; g1.nhp = (int)n;
-  if (h->mixed) return launch_convert<float>(g1, src, stage, 0, h->stream, hook_fn, h);
-  CK(cudaMemcpyAsync(stage, src, n * 16, cudaMemcpyDeviceToDevice, h->stream));
-  return 0;
+int pack_rows(gt_handle* h, void* field, int to_working) {
+  if (h->mixed) return launch_pack_rows<float>(h->g, h->stage, field, to_working, h->stream, hook_fn, h);
+  return launch_pack_rows<double>(h->g, h->stage, field, to_working, h->stream, hook_fn, h);
 }
+
+size_t real_bytes(const Geom& g) { return (size_t)g.nx * g.ny * g.nz * 8; }
 
 int upload_spec(gt_handle* h, const double* host, void* dst) {
-  const Geom& g = h->g;
-  CK(cudaMemcpy2DAsync(h->stage, (size_t)g.nhp * 16, host, (size_t)g.nh * 16, (size_t)g.nh * 16,
-                       (size_t)g.ny * g.nz, cudaMemcpyHostToDevice, h->stream));
-  CKI(to_working(h, h->stage, dst, g.field_elems()));
+  CK(cudaMemcpyAsync(h->stage, host, spec_bytes(h->g), cudaMemcpyHostToDevice, h->stream));
+  CKI(pack_rows(h, dst, 1));
   return GT_OK;
 }
 
 int download_spec(gt_handle* h, const void* src, double* host) {
-  const Geom& g = h->g;
-  CKI(from_working(h, src, h->stage, g.field_elems()));
-  CK(cudaMemcpy2DAsync(host, (size_t)g.nh * 16, h->stage, (size_t)g.nhp * 16, (size_t)g.nh * 16,
-                       (size_t)g.ny * g.nz, cudaMemcpyDeviceToHost, h->stream));
+  CKI(pack_rows(h, const_cast<void*>(src), 0));
+  CK(cudaMemcpyAsync(host, h->stage, spec_bytes(h->g), cudaMemcpyDeviceToHost, h->stream));
   return GT_OK;
 }
 
+// Real fields: FP64 ones are the host's layout already.
 int upload_real(gt_handle* h, const double* host, void* dst) {
   const Geom& g = h->g;
   const size_t n = (size_t)g.nx * g.ny * g.nz;
-  CK(cudaMemcpyAsync(h->stage, host, n * 8, cudaMemcpyHostToDevice, h->stream));
-  CKI(to_working(h, h->stage, dst, n / 2));
+  CK(cudaMemcpyAsync(h->mixed ? h->stage : dst, host, n * 8, cudaMemcpyHostToDevice, h->stream));
+  if (h->mixed) CKI(convert_real(h, h->stage, dst, n / 2, 1));
   return GT_OK;
 }
 
 int download_real(gt_handle* h, const void* src, double* host) {
   const Geom& g = h->g;
   const size_t n = (size_t)g.nx * g.ny * g.nz;
-  CKI(from_working(h, src, h->stage, n / 2));
-  CK(cudaMemcpyAsync(host, h->stage, n * 8, cudaMemcpyDeviceToHost, h->stream));
+  if (h->mixed) CKI(convert_real(h, src, h->stage, n / 2, 0));
+  CK(cudaMemcpyAsync(host, h->mixed ? h->stage : src, n * 8, cudaMemcpyDeviceToHost, h->stream));
   return GT_OK;
 }
 
@@ -611,6 +607,7 @@ int gt_get_state(gt_handle* h, double* bx, double* by, double* bz) {
   int rc = set_dev(h);
   if (rc) return rc;
   double* dst[3] = {bx, by, bz};
+  prefault(dst, 3, spec_bytes(h->g));
   for (int c = 0; c < 3; ++c) {
     if ((rc = download_spec(h, h->b[c], dst[c]))) return rc;
     CK(cudaStreamSynchronize(h->stream));   // the staging buffer is reused
@@ -669,6 +666,7 @@ int gt_nonlinear(gt_handle* h, const double* ax, const double* ay, const double*
     if ((rc = upload_spec(h, src[c], h->c[c]))) return rc;
   CKI(nlt(h, h->c, h->b, h->c, kNltOnly));
   double* dst[3] = {nx_out, ny_out, nz_out};
+  prefault(dst, 3, spec_bytes(h->g));
   for (int c = 0; c < 3; ++c) {
     if ((rc = download_spec(h, h->c[c], dst[c]))) return rc;
     CK(cudaStreamSynchronize(h->stream));
@@ -744,6 +742,7 @@ int gt_fft_dir(gt_handle* h, const double* real_in, double* spec_out) {
   if (rc) return rc;
   if ((rc = upload_real(h, real_in, h->w[1]))) return rc;
   CKI(fft_dir_dev(h, h->w[1], h->w[0]));
+  prefault(&spec_out, 1, spec_bytes(h->g));
   if ((rc = download_spec(h, h->w[0], spec_out))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return GT_OK;
@@ -755,6 +754,7 @@ int gt_fft_inv(gt_handle* h, const double* spec_in, double* real_out) {
   if (rc) return rc;
   if ((rc = upload_spec(h, spec_in, h->w[0]))) return rc;
   CKI(fft_inv_dev(h, h->w[0], h->w[1]));
+  prefault(&real_out, 1, real_bytes(h->g));
   if ((rc = download_real(h, h->w[1], real_out))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return GT_OK;
@@ -768,6 +768,7 @@ int gt_velocity(gt_handle* h, double* ux, double* uy, double* uz) {
   if ((rc = copy_fields(h, u, h->b))) return rc;
   CKI(point(h, u, 0, nullptr, 0));                        // curl (main.f90:195)
   double* dst[3] = {ux, uy, uz};
+  prefault(dst, 3, real_bytes(h->g));
   for (int c = 0; c < 3; ++c) {                           // fft_inv x3 (main.f90:197-199)
     CKI(fft_inv_dev(h, u[c], h->w[0]));
     if ((rc = download_real(h, h->w[0], dst[c]))) return rc;

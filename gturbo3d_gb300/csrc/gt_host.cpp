@@ -17,6 +17,9 @@
 #include <unordered_set>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "gt_internal.h"
 
 namespace gt {
@@ -270,6 +273,48 @@ bool entries_unique(const ForceEntry* e, size_t n) {
     if (!seen.insert(key).second) return false;
   }
   return true;
+}
+
+// Faults in the pages of host result arrays ahead of a device copy.  A copy
+// into untouched pages takes their faults one by one from the device (25 GB/s;
+// a fresh NumPy array is untouched), into present ones it runs at the link's
+// rate; the faults are taken here by several threads while the device still
+// computes.  Contents are not changed (MADV_POPULATE_WRITE), and a kernel
+// without it leaves everything as it was.  Ten FP64 steps at 256^3 and the state
+// (400 MB): 49.8 -> 41.6 ms; below 48 MB starting the threads costs more than
+// the faults (two transforms with 17 MB results 3.34 -> 3.70 ms).
+void prefault(double* const* dst, int n, size_t bytes) {
+  constexpr int kPopulateWrite = 23;          // MADV_POPULATE_WRITE, Linux 5.14
+  constexpr size_t kPart = (size_t)8 << 20;   // one thread's share at least
+  if (n * bytes < 6 * kPart) return;
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  struct Range {
+    uintptr_t a;
+    size_t len;
+  };
+  std::atomic<size_t> next{0};
+  try {
+    std::vector<Range> parts;
+    for (int k = 0; k < n; ++k) {
+      // whole pages inside the array only
+      const uintptr_t a = ((uintptr_t)dst[k] + page - 1) / page * page, b = ((uintptr_t)dst[k] + bytes) / page * page;
+      for (uintptr_t p = a; p < b; p += kPart) parts.push_back({p, std::min<size_t>(kPart, b - p)});
+    }
+    auto work = [&] {
+      for (size_t i; (i = next.fetch_add(1)) < parts.size();)
+        if (madvise(reinterpret_cast<void*>(parts[i].a), parts[i].len, kPopulateWrite) != 0) return;
+    };
+    const size_t nt = std::min<size_t>({parts.size(), std::max(1u, std::thread::hardware_concurrency()), (size_t)16});
+    std::vector<std::thread> pool;
+    pool.reserve(nt);
+    try {
+      for (size_t t = 1; t < nt; ++t) pool.emplace_back(work);
+    } catch (...) {   // fewer threads than wanted
+    }
+    work();
+    for (auto& t : pool) t.join();
+  } catch (...) {     // no memory for the bookkeeping: the copy takes the faults itself
+  }
 }
 
 }  // namespace gt

@@ -57,6 +57,8 @@ float rann(int32_t& irand);
 void draw_forcing(const gt_params& p, const HostTables& t, int32_t& seed,
                   std::vector<ForceEntry>& out);
 bool entries_unique(const ForceEntry* e, size_t n);
+// Faults in n host arrays of `bytes` each before device results are copied there.
+void prefault(double* const* dst, int n, size_t bytes);
 
 // ---- device side --------------------------------------------------------
 
@@ -207,11 +209,15 @@ int launch_force_batch(const Geom& g, void* const b[3], const Batch<R>& bt, cons
 template <typename R>
 int launch_force_indexed(const Geom& g, void* const b[3], const ForceEntry* base, int n,
                          const int* step, void* stream, LaunchHook hook, void* hctx);
-// Field conversions between the device FP64 staging layout [nz][ny][nhp]
-// double2 and the working precision.
+// Conversion of g.field_elems() complex values between FP64 staging and the
+// working precision.
 template <typename R>
 int launch_convert(const Geom& g, const void* src, void* dst, int to_working, void* stream,
                    LaunchHook hook, void* hctx);
+// A field's rows <-> packed FP64 rows [nz][ny][nh] (the host layout).
+template <typename R>
+int launch_pack_rows(const Geom& g, void* packed, void* field, int to_working, void* stream, LaunchHook hook,
+                     void* hctx);
 // Plain 3D transforms of one field (real layout [nz][ny][nx] in w-buffers).
 template <typename R>
 int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* spec, void* real_out,

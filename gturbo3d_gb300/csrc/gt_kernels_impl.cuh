@@ -2036,6 +2036,30 @@ __global__ void k_convert(const double2* __restrict__ s64, Cplx<R>* __restrict__
   }
 }
 
+// A field's rows between the padded working layout and the host's packed FP64
+// one ([rows][nh]), one warp a row: the host copy is then one contiguous
+// transfer.  A strided cudaMemcpy2D of 4112-byte rows into pageable memory ran
+// at 1 GB/s (3.1 s for the three fields of 512^3).
+template <typename R>
+__global__ void __launch_bounds__(256)
+k_pack_rows(double2* __restrict__ packed, Cplx<R>* __restrict__ f, size_t rows, int nh, int nhp, int to_working) {
+  const int lane = threadIdx.x & 31;
+  const size_t nw = (size_t)gridDim.x * 8;
+  for (size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += nw) {
+    double2* p = packed + row * nh;
+    Cplx<R>* q = f + row * nhp;
+    for (int X = lane; X < nh; X += 32) {
+      if (to_working) {
+        const double2 v = p[X];
+        q[X] = Cplx<R>{(R)v.x, (R)v.y};
+      } else {
+        const Cplx<R> v = q[X];
+        p[X] = double2{(double)v.x, (double)v.y};
+      }
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Diagnostics.  Each warp walks whole (y,z) rows; along a row |k| grows with
 // kx, so the shell index is non-decreasing and lanes add to warp-private
@@ -3013,6 +3037,19 @@ int launch_convert(const Geom& g, const void* src, void* dst, int to_working, vo
 }
 
 template <typename R>
+int launch_pack_rows(const Geom& g, void* packed, void* field, int to_working, void* stream, LaunchHook hook,
+                     void* hctx) {
+  const size_t rows = (size_t)g.ny * g.nz;
+  const int blocks = (int)std::min<size_t>((rows + 7) / 8, 152 * 16);
+  GT_HOOK(kKConvert, true);
+  k_pack_rows<R><<<blocks, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<double2*>(packed),
+                                                           reinterpret_cast<Cplx<R>*>(field), rows, g.nh, g.nhp,
+                                                           to_working);
+  GT_HOOK(kKConvert, false);
+  return (int)cudaGetLastError();
+}
+
+template <typename R>
 int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* spec, void* real_out,
                    void* const w[6], void* stream, LaunchHook hook, void* hctx) {
   int rc = set_smem_attrs<R>();
@@ -3243,6 +3280,7 @@ const char* kernel_kind_name(int k) {
                                      LaunchHook, void*);                                        \
   template int launch_convert<R>(const Geom&, const void*, void*, int, void*, LaunchHook,      \
                                  void*);                                                        \
+  template int launch_pack_rows<R>(const Geom&, void*, void*, int, void*, LaunchHook, void*);   \
   template int launch_fft_inv<R>(const Geom&, const DevTables<R>&, void*, void*, void* const*, \
                                  void*, LaunchHook, void*);                                     \
   template int launch_fft_dir<R>(const Geom&, const DevTables<R>&, const void*, void*,         \

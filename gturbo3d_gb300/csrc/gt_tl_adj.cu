@@ -202,6 +202,7 @@ int tl_or_adj(gt_handle* h, const double* in[3], double* out[3], bool adjoint) {
   }
   rc = adjoint ? S.adj(b, x, y) : S.tl(b, x, y);
   if (rc) return rc;
+  prefault(out, 3, spec_bytes(h->g));
   for (int c = 0; c < 3; ++c) {
     if ((rc = download_spec(h, y.p[c], out[c]))) return rc;
     CK(cudaStreamSynchronize(h->stream));
@@ -290,6 +291,7 @@ int gradient(gt_handle* h, int nsteps, int32_t seed, int K, double kmin, double*
     }
   }
   copy3(state, b0);
+  prefault(gout, 3, spec_bytes(h->g));
   CK(cudaStreamSynchronize(h->stream));
   h->state_in_k = was_in_k;
   for (int c = 0; c < 3; ++c) {
