@@ -3,6 +3,7 @@
 // initial-state / output paths.  See include/gturbo_gb.h for the contract.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -256,10 +257,11 @@ void free_handle(gt_handle* h) {
   }
   for (auto e : h->pool) cudaEventDestroy(e);
   for (int i = 0; i < 2; ++i) {
-    if (h->d_force[i]) cudaFree(h->d_force[i]);
     if (h->h_force[i]) cudaFreeHost(h->h_force[i]);
     if (h->force_copied[i]) cudaEventDestroy(h->force_copied[i]);
   }
+  if (h->sg.exec) cudaGraphExecDestroy(h->sg.exec);
+  if (h->d_force) cudaFree(h->d_force);
   if (h->fields_mem && h->owns_fields) cudaFree(h->fields_mem);
   if (h->stage) cudaFree(h->stage);
   if (h->tab_mem) cudaFree(h->tab_mem);
@@ -409,46 +411,150 @@ int copy_fields(gt_handle* h, void* const dst[3], void* const src[3]) {
   return GT_OK;
 }
 
-int ensure_force_cap(gt_handle* h, int slot, size_t n) {
-  if (h->force_cap[slot] >= n) return GT_OK;
-  size_t cap = 256;
-  while (cap < n) cap *= 2;
+// Room for `bytes` of forcing in the device buffer and pinned slot `slot`.
+int ensure_force_cap(gt_handle* h, int slot, size_t bytes) {
+  if (h->d_force_cap >= bytes && h->h_force_cap[slot] >= bytes) return GT_OK;
+  size_t cap = (size_t)1 << 16;
+  while (cap < bytes) cap *= 2;
   CK(cudaStreamSynchronize(h->stream));
-  if (h->d_force[slot]) cudaFree(h->d_force[slot]);
-  if (h->h_force[slot]) cudaFreeHost(h->h_force[slot]);
-  h->d_force[slot] = nullptr;
-  h->h_force[slot] = nullptr;
-  h->force_cap[slot] = 0;
-  CK(cudaMalloc(&h->d_force[slot], cap * sizeof(ForceEntry)));
-  CK(cudaMallocHost(&h->h_force[slot], cap * sizeof(ForceEntry)));
-  h->force_cap[slot] = cap;
+  if (h->d_force_cap < bytes) {
+    if (h->sg.exec) cudaGraphExecDestroy(h->sg.exec);   // holds the buffer's address
+    h->sg.exec = nullptr;
+    if (h->d_force) cudaFree(h->d_force);
+    h->d_force = nullptr;
+    h->d_force_cap = 0;
+    CK(cudaMalloc(&h->d_force, cap));
+    h->d_force_cap = cap;
+  }
+  if (h->h_force_cap[slot] < bytes) {
+    if (h->h_force[slot]) cudaFreeHost(h->h_force[slot]);
+    h->h_force[slot] = nullptr;
+    h->h_force_cap[slot] = 0;
+    CK(cudaMallocHost(&h->h_force[slot], cap));
+    h->h_force_cap[slot] = cap;
+  }
   return GT_OK;
+}
+
+// Grids whose step's kernels take less time than their 11 launches, about 9 us
+// each from this host: the step is replayed as one graph (mixed, us a step: 16^3
+// 113 -> 92, 64^3 103 -> 75, 128^3 182 -> 155).  At 256^3 the kernels take 0.85 ms.
+constexpr size_t kGraphPoints = (size_t)1 << 22;
+// A graph costs about as much to build as 16 steps take to launch.
+constexpr int64_t kGraphAfter = 16;
+
+std::vector<int> graph_key(const gt_handle* h, int pr, bool forced) {
+  const PassTuning& p = h->pm;
+  return {pr, forced, p.y_tx, p.z_tx, p.y_pairs, p.y_prefetch, p.x_fused, p.fuse_stage, p.z_split, p.overlap,
+          p.zf_pipe, p.slab_pipe, p.z_tma, p.z_cluster};
+}
+
+// Whether this call's steps go through the step graph; builds it when due.
+// Anything in the way (profiling, the caller's own capture, a failed capture)
+// leaves the direct launches.
+bool use_step_graph(gt_handle* h, int nsteps, int pr, bool forced) {
+  auto& sg = h->sg;
+  const Geom& g = h->g;
+  if (sg.broken || h->prof || (size_t)g.nx * g.ny * g.nz > kGraphPoints) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+  const std::vector<int> key = graph_key(h, pr, forced);
+  if (key != sg.key) {
+    if (sg.exec) {
+      cudaStreamSynchronize(h->stream);
+      cudaGraphExecDestroy(sg.exec);
+    }
+    sg.exec = nullptr;
+    sg.key = key;
+    sg.steps = 0;
+  }
+  if (sg.exec) return true;
+  // the first step with these passes runs directly, which also loads the
+  // kernels and their attributes outside a capture
+  if (sg.steps == 0 || sg.steps + nsteps < kGraphAfter) return false;
+  const int64_t before = h->launches;
+  if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
+    cudaGetLastError();
+    sg.broken = true;
+    return false;
+  }
+  int rc = rk2_nlts(h, pr);
+  if (!rc && forced) {
+    auto* head = reinterpret_cast<ForceHead*>(h->d_force);
+    rc = h->mixed ? launch_force_head<float>(g, h->b, head, h->stream, hook_fn, h)
+                  : launch_force_head<double>(g, h->b, head, h->stream, hook_fn, h);
+  }
+  cudaGraph_t graph = nullptr;
+  const cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
+  sg.launches = h->launches - before;
+  h->launches = before;
+  if (rc || ce != cudaSuccess || cudaGraphInstantiate(&sg.exec, graph, 0) != cudaSuccess) {
+    cudaGetLastError();
+    sg.exec = nullptr;
+    sg.broken = true;
+  }
+  if (graph) cudaGraphDestroy(graph);
+  return sg.exec != nullptr;
+}
+
+// Whether no step's entries name a mode twice.  Steps of one forcing have the
+// same modes: those are looked at once.
+bool steps_unique(int nsteps, const std::vector<ForceEntry>& all, const std::vector<size_t>& offs) {
+  const size_t n0 = offs[1] - offs[0];
+  if (!entries_unique(all.data() + offs[0], n0)) return false;
+  for (int s = 1; s < nsteps; ++s) {
+    const ForceEntry *e = all.data() + offs[s], *e0 = all.data() + offs[0];
+    const size_t n = offs[s + 1] - offs[s];
+    bool same = n == n0;
+    for (size_t i = 0; same && i < n; ++i) same = e[i].x == e0[i].x && e[i].y == e0[i].y && e[i].z == e0[i].z;
+    if (!same && !entries_unique(e, n)) return false;
+  }
+  return true;
 }
 
 // Enqueues nsteps RK2 steps; entries[s] are the forcing adds of step s.
 int run_steps(gt_handle* h, int nsteps, const std::vector<ForceEntry>& all,
               const std::vector<size_t>& offs) {
-  const int slot = h->force_slot;
-  h->force_slot ^= 1;
+  if (nsteps <= 0) return GT_OK;
+  const int pr = use_pruning(h) ? 1 : 0;
+  const bool forced = !all.empty();
+  const bool unique = !forced || steps_unique(nsteps, all, offs);
+  bool even = true;   // as many entries in every step
+  for (int s = 1; forced && s < nsteps; ++s) even = even && offs[s + 1] - offs[s] == offs[1] - offs[0];
   const ForceEntry* dent = nullptr;
-  if (!all.empty()) {
-    int rc = ensure_force_cap(h, slot, all.size());
+  if (forced) {
+    const int slot = h->force_slot;
+    h->force_slot ^= 1;
+    const size_t bytes = sizeof(ForceHead) + all.size() * sizeof(ForceEntry);
+    int rc = ensure_force_cap(h, slot, bytes);
     if (rc) return rc;
     CK(cudaEventSynchronize(h->force_copied[slot]));   // previous user of this slot is done
-    std::memcpy(h->h_force[slot], all.data(), all.size() * sizeof(ForceEntry));
-    CK(cudaMemcpyAsync(h->d_force[slot], h->h_force[slot], all.size() * sizeof(ForceEntry),
-                       cudaMemcpyHostToDevice, h->stream));
+    auto* head = reinterpret_cast<ForceHead*>(h->h_force[slot]);
+    *head = ForceHead{};
+    head->n = (int)(offs[1] - offs[0]);
+    std::memcpy(head + 1, all.data(), all.size() * sizeof(ForceEntry));
+    // in stream order behind the steps that read the buffer
+    CK(cudaMemcpyAsync(h->d_force, head, bytes, cudaMemcpyHostToDevice, h->stream));
     CK(cudaEventRecord(h->force_copied[slot], h->stream));
-    dent = h->d_force[slot];
+    dent = reinterpret_cast<const ForceEntry*>(h->d_force + sizeof(ForceHead));
   }
-  const int pr = use_pruning(h) ? 1 : 0;
   for (int s = 0; s < nsteps; ++s) {
+    const size_t n = offs[s + 1] - offs[s];
+    if (unique && even && s < 128 && use_step_graph(h, nsteps - s, pr, forced)) {
+      if (s > 0 && forced)   // the entries' head says which step comes next
+        CK(cudaMemsetAsync(h->d_force + offsetof(ForceHead, step), s, 1, h->stream));
+      for (; s < nsteps; ++s) {
+        CK(cudaGraphLaunch(h->sg.exec, h->stream));
+        h->launches += h->sg.launches;
+      }
+      break;
+    }
     CKI(rk2_nlts(h, pr));                      // main.f90:124-146
     if (dent) {                               // main.f90:149
-      const size_t n = offs[s + 1] - offs[s];
-      const bool serial = !entries_unique(all.data() + offs[s], n);
+      const bool serial = !unique && !entries_unique(all.data() + offs[s], n);
       CKI(force(h, dent + offs[s], (int)n, serial ? 1 : 0));
     }
+    ++h->sg.steps;
   }
   return GT_OK;
 }
@@ -621,15 +727,20 @@ int gt_rk2_step(gt_handle* h, int32_t nsteps, int32_t* seed_inout) {
   if (forced && !seed_inout) return GT_EINVAL;
   int rc = set_dev(h);
   if (rc) return rc;
-  std::vector<ForceEntry> all;
-  std::vector<size_t> offs(1, 0);
+  // in chunks, so that the host draws the next steps' forcing while the device
+  // works on the last ones
+  constexpr int kChunk = 32;
   int32_t seed = seed_inout ? *seed_inout : 0;
-  for (int s = 0; s < nsteps; ++s) {
-    if (forced) draw_forcing(h->p, h->ht, seed, all);
-    offs.push_back(all.size());
+  for (int done = 0; done < nsteps; done += kChunk) {
+    const int n = std::min(kChunk, nsteps - done);
+    std::vector<ForceEntry> all;
+    std::vector<size_t> offs(1, 0);
+    for (int s = 0; s < n; ++s) {
+      if (forced) draw_forcing(h->p, h->ht, seed, all);
+      offs.push_back(all.size());
+    }
+    if ((rc = run_steps(h, n, all, offs))) return rc;
   }
-  rc = run_steps(h, nsteps, all, offs);
-  if (rc) return rc;
   CK(cudaGetLastError());
   if (seed_inout) *seed_inout = seed;
   return GT_OK;

@@ -51,12 +51,23 @@ struct gt_handle {
   void* tab_mem = nullptr;
   gt::DevTables<double> t64{};
   gt::DevTables<float> t32{};
-  // forcing entries: double-buffered pinned staging and device buffers
-  gt::ForceEntry* d_force[2]{};
-  gt::ForceEntry* h_force[2]{};
-  size_t force_cap[2]{};
+  // forcing entries of the steps in one run_steps call: the device buffer is
+  // refilled in stream order, the pinned staging is double-buffered
+  char* d_force = nullptr;     // gt::ForceHead, then the entries
+  size_t d_force_cap = 0;
+  char* h_force[2]{};
+  size_t h_force_cap[2]{};
   cudaEvent_t force_copied[2]{};
   int force_slot = 0;
+  // small grids: one RK2 step as a CUDA graph (run_steps), rebuilt when the
+  // passes it was captured with change
+  struct {
+    cudaGraphExec_t exec = nullptr;
+    std::vector<int> key;        // pruning, forcing and the launch-shape knobs it holds
+    int64_t launches = 0;        // kernels a replay launches
+    int64_t steps = 0;           // steps taken with this key
+    bool broken = false;         // capture or instantiation failed once
+  } sg;
   double* d_partials = nullptr;
   int npartials = 0;
   double* d_result = nullptr;

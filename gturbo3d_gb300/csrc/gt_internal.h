@@ -60,6 +60,12 @@ bool entries_unique(const ForceEntry* e, size_t n);
 // Faults in n host arrays of `bytes` each before device results are copied there.
 void prefault(double* const* dst, int n, size_t bytes);
 
+// Resident forcing of a graph-replayed step: n entries a step follow the head;
+// the scatter kernel adds those of step `step` and advances it.
+struct ForceHead {
+  int32_t n, step, pad[14];
+};
+
 // ---- device side --------------------------------------------------------
 
 // Layout of one spectral field on the device: [nz][ny][nhp] complex with the
@@ -209,6 +215,9 @@ int launch_force_batch(const Geom& g, void* const b[3], const Batch<R>& bt, cons
 template <typename R>
 int launch_force_indexed(const Geom& g, void* const b[3], const ForceEntry* base, int n,
                          const int* step, void* stream, LaunchHook hook, void* hctx);
+// Forcing of step head->step from resident entries, then ++head->step.
+template <typename R>
+int launch_force_head(const Geom& g, void* const b[3], ForceHead* head, void* stream, LaunchHook hook, void* hctx);
 // Conversion of g.field_elems() complex values between FP64 staging and the
 // working precision.
 template <typename R>

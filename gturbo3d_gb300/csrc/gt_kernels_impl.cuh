@@ -2016,6 +2016,29 @@ __global__ void k_force_batch(Ptr6 b, const ForceEntry* __restrict__ base, const
   }
 }
 
+// Forcing of a captured step (one block): the step's entries, then the counter.
+constexpr int kForceThreads = 128;
+template <typename R>
+__global__ void __launch_bounds__(kForceThreads)
+k_force_head(Ptr6 b, ForceHead* head, Geom g) {
+  using C = Cplx<R>;
+  const int n = head->n, step = head->step;
+  const ForceEntry* e = reinterpret_cast<const ForceEntry*>(head + 1) + (size_t)step * n;
+  for (int m = threadIdx.x; m < n; m += kForceThreads) {
+    const ForceEntry en = e[m];
+    const size_t o = ((size_t)en.z * g.ny + en.y) * g.nhp + en.x;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (!(en.mask & (1 << c))) continue;
+      C* p = reinterpret_cast<C*>(b.at(c));
+      const C v = p[o];
+      p[o] = C{v.x + (R)en.inc[2 * c], v.y + (R)en.inc[2 * c + 1]};
+    }
+  }
+  __syncthreads();   // everyone has read the step
+  if (threadIdx.x == 0) head->step = step + 1;
+}
+
 static __global__ void k_step_inc(int* step) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *step += 1;
 }
@@ -3004,6 +3027,16 @@ int launch_force_indexed(const Geom& g, void* const b[3], const ForceEntry* base
 }
 
 template <typename R>
+int launch_force_head(const Geom& g, void* const b[3], ForceHead* head, void* stream, LaunchHook hook, void* hctx) {
+  Ptr6 pb{};
+  for (int i = 0; i < 3; ++i) pb.p[i] = b[i];
+  GT_HOOK(kKForce, true);
+  k_force_head<R><<<1, kForceThreads, 0, (cudaStream_t)stream>>>(pb, head, g);
+  GT_HOOK(kKForce, false);
+  return (int)cudaGetLastError();
+}
+
+template <typename R>
 int launch_force_batch(const Geom& g, void* const b[3], const Batch<R>& bt, const ForceEntry* base,
                        const int* count, int nmax, int nsteps, const int* step, void* stream,
                        LaunchHook hook, void* hctx) {
@@ -3275,6 +3308,7 @@ const char* kernel_kind_name(int k) {
                                LaunchHook, void*);                                              \
   template int launch_force_indexed<R>(const Geom&, void* const*, const ForceEntry*, int,      \
                                        const int*, void*, LaunchHook, void*);                  \
+  template int launch_force_head<R>(const Geom&, void* const*, ForceHead*, void*, LaunchHook, void*); \
   template int launch_force_batch<R>(const Geom&, void* const*, const Batch<R>&,                \
                                      const ForceEntry*, const int*, int, int, const int*, void*, \
                                      LaunchHook, void*);                                        \
