@@ -790,13 +790,14 @@ int gt_diagnostics(gt_handle* h, gt_diag* out, double* ek, double* ek2d, double*
   int rc = set_dev(h);
   if (rc) return rc;
   const Geom& g = h->g;
-  if (flux) CKI(nlt(h, h->b, h->b, h->c, kNltOnly));   // N1 = nlt(b) (main.f90:131-136)
+  const int pr = use_pruning(h) ? 1 : 0;   // state (and N1) zero outside the kept set
+  if (flux) CKI(nlt(h, h->b, h->b, h->c, kNltOnly, pr));   // N1 = nlt(b) (main.f90:131-136)
   const int nblk = diag_blocks(g);
   if (h->mixed)
-    CKI(launch_diag<float>(g, h->t32, h->b, flux ? h->c : nullptr, h->p.nu, h->p.alpnu, h->p.mu,
+    CKI(launch_diag<float>(g, h->t32, h->b, flux ? h->c : nullptr, pr, h->p.nu, h->p.alpnu, h->p.mu,
                            h->p.alpmu, h->d_partials, nblk, h->d_result, h->stream, hook_fn, h));
   else
-    CKI(launch_diag<double>(g, h->t64, h->b, flux ? h->c : nullptr, h->p.nu, h->p.alpnu, h->p.mu,
+    CKI(launch_diag<double>(g, h->t64, h->b, flux ? h->c : nullptr, pr, h->p.nu, h->p.alpnu, h->p.mu,
                             h->p.alpmu, h->d_partials, nblk, h->d_result, h->stream, hook_fn, h));
   CK(cudaMemcpyAsync(h->h_result, h->d_result, (size_t)h->nresult * sizeof(double),
                      cudaMemcpyDeviceToHost, h->stream));

@@ -243,7 +243,7 @@ int launch_point(const Geom& g, const DevTables<R>& tb, void* const a[3], int op
 // Diagnostics: per-CTA partials then a fixed-order final reduction.
 constexpr int kDiagScalars = 20;  // 9 energy, 9 enstrophy, helicity, nonfinite
 template <typename R>
-int launch_diag(const Geom& g, const DevTables<R>& tb, void* const b[3], void* const n1[3],
+int launch_diag(const Geom& g, const DevTables<R>& tb, void* const b[3], void* const n1[3], int prune,
                 double nu, double alpnu, double mu, double alpmu, double* partials, int nblocks,
                 double* result /* kDiagScalars + 3*nbin */, void* stream, LaunchHook hook,
                 void* hctx);
