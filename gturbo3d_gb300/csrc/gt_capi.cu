@@ -119,6 +119,12 @@ int upload_tables(gt_handle* h, DevTables<R>& t) {
   const size_t o_fkx = putR(ht.fkx), o_fky = putR(ht.fky), o_fkz = putR(ht.fkz);
   const size_t o_fkxs = putR(ht.fkxs), o_fkys = putR(ht.fkys), o_fkzs = putR(ht.fkzs);
   const size_t o_emk = putR(ht.emk_by_k2 ? ht.emk_k2 : ht.emk_full);
+  size_t o_ik2 = 0;
+  if (sizeof(R) == 8 && ht.emk_by_k2) {
+    std::vector<double> q(ht.emk_k2.size(), 1.0);
+    for (size_t k = 1; k < q.size(); ++k) q[k] = 1.0 / (double)k;
+    o_ik2 = putR(q);
+  }
   const size_t o_xcut = put(ht.xcut.data(), ht.xcut.size() * sizeof(int32_t));
   // Each axis: the full table tw[m] = exp(-2 pi i m / L), m < L, followed by
   // the per-stage table of the Stockham line transform (tw_stage_offset in
@@ -223,6 +229,7 @@ int upload_tables(gt_handle* h, DevTables<R>& t) {
   t.fkzs = dptr<const R>(mem, o_fkzs);
   t.emk = dptr<const R>(mem, o_emk);
   t.emk_by_k2 = ht.emk_by_k2 ? 1 : 0;
+  t.ik2 = o_ik2 ? dptr<const R>(mem, o_ik2) : nullptr;
   t.xcut = dptr<const int32_t>(mem, o_xcut);
   t.twx = dptr<const void>(mem, o_twx);
   t.twy = dptr<const void>(mem, o_twy);

@@ -15,10 +15,9 @@ template <int LGL> constexpr int fx_tile() { return kFxTileThreads >> (LGL - 3);
 static inline int fx_lg_tile(int lgl) { return 11 - lgl; }
 
 // Slots of a strided pass: lines are the tile's columns, x = threadIdx % TX.
-template <int LGL> using FxTileRed = FxRed<fx_tile<LGL>(), 32, 1>;
-template <int LGL> __device__ __forceinline__ FxTileRed<LGL> fx_red_tile(unsigned* slots, int x, int t) {
-  constexpr int TX = fx_tile<LGL>();
-  return FxTileRed<LGL>{slots, x & (kFxLines - 1), TX >= 32 || (int)(threadIdx.x & 31) < TX, t == 0};
+template <int TX> using FxTileRed = FxRed<TX, 32, 1>;
+template <int TX> __device__ __forceinline__ FxTileRed<TX> fx_red_tile(unsigned* slots, int x, int t) {
+  return FxTileRed<TX>{slots, x & (kFxLines - 1), TX >= 32 || (int)(threadIdx.x & 31) < TX, t == 0};
 }
 // Slots of an x pass: lines are groups of T consecutive threads.
 template <int LGN, int NQ> using FxRowRed = FxRed<1, ((1 << (LGN - 3)) < 32 ? (1 << (LGN - 3)) : 32), NQ>;
@@ -31,25 +30,28 @@ template <int LGN, int NQ> __device__ __forceinline__ FxRowRed<LGN, NQ> fx_red_r
 // point.  Each output line is formed from the input columns read again (after
 // the first read, from L1 or L2), so a block needs one shared region and 24
 // warps share an SM; with u_y and u_z parked in two more regions 16 do
-// (1.99 against 1.91 ms at 512^3).
+// (1.99 against 1.91 ms at 512^3).  split: one output line per block
+// (blockIdx.z = 6 member + line in a full launch, line in a pruned one), where
+// the tiles alone leave SMs idle.
 // ---------------------------------------------------------------------------
 template <int LGZ>
 __global__ void __launch_bounds__(kFxTileThreads, 3)
 k_fx_zinv(Ptr6 a, Ptr6 w, DevTables<double> tb, Geom g, int pruned, const int32_t* __restrict__ tiles,
-          FxExp ex, long long fxs, long long mstride) {
+          int split, FxExp ex, long long fxs, long long mstride) {
   using C = double2;
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ unsigned slots[FxTileRed<LGZ>::kSlots];
-  __shared__ int emax[6][kFxLines];
   constexpr int TX = fx_tile<LGZ>();
+  __shared__ unsigned slots[FxTileRed<TX>::kSlots];
+  __shared__ int emax[6][kFxLines];
   const int x = threadIdx.x % TX, t = threadIdx.x / TX;
   int tile = blockIdx.x, y = blockIdx.y;
   if (pruned) {
     tile = tiles[2 * blockIdx.x];
     y = tiles[2 * blockIdx.x + 1];
   }
-  const unsigned mem = pruned ? blockIdx.y : blockIdx.z;
+  const unsigned mem = pruned ? blockIdx.y : (split ? blockIdx.z / 6 : blockIdx.z);
+  const int f0 = split ? (int)(blockIdx.z % 6) : 0, f1 = split ? f0 + 1 : 6;
   const int X = tile * TX + x;
   const int ylim = pruned ? tb.xcut[y] : g.nh;
   const bool valid = X < ylim;
@@ -57,7 +59,7 @@ k_fx_zinv(Ptr6 a, Ptr6 w, DevTables<double> tb, Geom g, int pruned, const int32_
   const size_t plane = (size_t)g.ny * g.nhp;
   const size_t base = (size_t)y * g.nhp + (valid ? X : 0) + member_offset(mstride, mem);
   const int4* tw = reinterpret_cast<const int4*>(tb.fwz);
-  auto red = fx_red_tile<LGZ>(slots, x, t);
+  auto red = fx_red_tile<TX>(slots, x, t);
   red.clear_all();
   for (int i = threadIdx.x; i < 6 * kFxLines; i += blockDim.x) (&emax[0][0])[i] = 0;
   __syncthreads();
@@ -65,7 +67,7 @@ k_fx_zinv(Ptr6 a, Ptr6 w, DevTables<double> tb, Geom g, int pruned, const int32_
   const double ky = tb.fky[y], kys = tb.fkys[y];
   const FxMem<LGZ, TX> mem_{reinterpret_cast<E*>(smraw) + x};
 #pragma unroll 1
-  for (int f = 0; f < 6; ++f) {
+  for (int f = f0; f < f1; ++f) {
     // the fields output f reads: u_0 <- (a1, a2), u_1 <- (a2, a0), u_2 <- (a0, a1); w_c <- a_c.
     // u_f = i (k1 p2 - k2 p1) with (k1, k2) the wavenumbers of the two other axes in cyclic order
     const C* p1 = reinterpret_cast<const C*>(a.at(f < 3 ? (f == 2 ? 0 : f + 1) : f - 3));
@@ -134,9 +136,9 @@ k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim
   using E = longlong2;
   constexpr int SIGN = (KIND == 0 || KIND == 2) ? +1 : -1;
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ unsigned slots[FxTileRed<LGL>::kSlots];
-  __shared__ int emax[KIND == 2 ? kFxLines : 1];
   constexpr int TX = fx_tile<LGL>();
+  __shared__ unsigned slots[FxTileRed<TX>::kSlots];
+  __shared__ int emax[KIND == 2 ? kFxLines : 1];
   const int x = threadIdx.x % TX, t = threadIdx.x / TX;
   const int X = blockIdx.x * TX + x;
   const bool valid = X < xlim;
@@ -144,7 +146,7 @@ k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim
   const int fi = blockIdx.z % nf, mem = blockIdx.z / nf, o = blockIdx.y;
   E* p = reinterpret_cast<E*>(f.at(fi));
   const size_t base = (size_t)o * (size_t)os + (valid ? X : 0) + member_offset(mstride, mem);
-  auto red = fx_red_tile<LGL>(slots, x, t);
+  auto red = fx_red_tile<TX>(slots, x, t);
   red.clear_all();
   const long long xo = mem * fxs;
   const int Xc = valid ? X : 0;
@@ -503,18 +505,89 @@ k_fx_xr2c(const double* __restrict__ real, void* specv, Geom g, const void* twv,
   }
 }
 
+// The spectral epilogue of pass 5 (nlt.f90:67-81, produ.f90:83-99,
+// trunc.f90:14-28, rkstep.f90:30-48 / 86-104) at one thread's own positions, from
+// the fixed-point transforms in three regions `reg` apart (exponents e).  The
+// FP64 pipe bounds it, so with a = v + i omega kz b the update e (e' b + d i k x
+// a / k^2) (e' = 1 or e) is formed with d k / k^2 as one vector, 1/k^2 comes from
+// a table where the integrating factor does, and only the modes that are written
+// are converted: 38 FP64 operations a mode instead of 61 with the division.
+// (e' e as one factor would save six more, but its rounding repeats every step:
+// 100 steps at 64^3 were off by 4.3e-15 instead of 0.9e-15.)
+template <int LGT, int TX>
+__device__ __forceinline__ void fx_epilogue(longlong2* __restrict__ sm, int reg, const int e[3], int t, int X, int y,
+                                            int ylim, size_t base, size_t plane, const Ptr6& bc, const Ptr6& out,
+                                            const DevTables<double>& tb, const Geom& g, int mode, int pruned) {
+  using C = double2;
+  constexpr int T = 1 << (LGT - 3);
+  const double kx = tb.fkx[X], ky = tb.fky[y];
+  const double kxys = tb.fkxs[X] + tb.fkys[y];
+  const int k2xy = tb.emk_by_k2 ? (int)kxys : 0;
+  const C* b0p = reinterpret_cast<const C*>(bc.p[0]);
+  const C* b1p = reinterpret_cast<const C*>(bc.p[1]);
+  const C* b2p = reinterpret_cast<const C*>(bc.p[2]);
+  const FxMem<LGT, TX> mem{sm};
+#pragma unroll 2
+  for (int i = 0; i < 8; ++i) {
+    const int z = t + i * T;
+    const int zlim = tb.xcut[(size_t)z * g.ny + y];   // kept modes of this row: X < zlim
+    if (X >= (pruned ? zlim : ylim)) continue;        // written columns: the kept ones, or all of the row's
+    const size_t o = (size_t)z * plane + base;
+    const C b0 = b0p[o], b1 = b1p[o], b2 = b2p[o];
+    const longlong2* const n = &mem.at(z);
+    const double kz = tb.fkz[z], okz = tb.omega * kz;
+    const bool zero_mode = (X == 0) && (y == 0) && (z == 0);
+    double em = 1.0, ik2;
+    if (tb.emk_by_k2) {
+      const int k2 = k2xy + (int)tb.fkzs[z];
+      ik2 = tb.ik2[k2];
+      if (mode != kNltOnly) em = tb.emk[k2];
+    } else {
+      ik2 = 1.0 / (kxys + tb.fkzs[z]);
+      if (mode != kNltOnly) em = tb.emk[((size_t)z * g.ny + y) * g.nh + X];
+    }
+    auto val = [&](int f, const C& b) {   // v + i omega kz b(t)
+      const longlong2 q = n[f * reg];
+      return C{fx_to_double(q.x, e[f]) - okz * b.y, fx_to_double(q.y, e[f]) + okz * b.x};
+    };
+    C a0 = val(0, b0), a1 = val(1, b1), a2 = val(2, b2);
+    if (tb.truncate && (zero_mode || X >= zlim)) a0 = a1 = a2 = C{0, 0};
+    C s0, s1, s2;
+    if (mode == kNltOnly) {
+      const double qx = kx * ik2, qy = ky * ik2, qz = kz * ik2;
+      s0 = C{-qy * a2.y + qz * a1.y, qy * a2.x - qz * a1.x};
+      s1 = C{-qz * a0.y + qx * a2.y, qz * a0.x - qx * a2.x};
+      s2 = C{-qx * a1.y + qy * a0.y, qx * a1.x - qy * a0.x};
+      if (zero_mode) { s0 = a0; s1 = a1; s2 = a2; }   // produ.f90:83
+    } else {
+      const double c = mode == kStage1 ? 1.0 : em;
+      const double d = ik2 * (mode == kStage1 ? tb.dt2 : tb.dt);
+      const double qx = kx * d, qy = ky * d, qz = kz * d;
+      s0 = C{em * (qz * a1.y + (c * b0.x - qy * a2.y)), em * (qy * a2.x + (c * b0.y - qz * a1.x))};
+      s1 = C{em * (qx * a2.y + (c * b1.x - qz * a0.y)), em * (qz * a0.x + (c * b1.y - qx * a2.x))};
+      s2 = C{em * (qy * a0.y + (c * b2.x - qx * a1.y)), em * (qx * a1.x + (c * b2.y - qy * a0.x))};
+      if (zero_mode) s0 = s1 = s2 = C{0, 0};          // rkstep.f90:44-48 / 100-104
+    }
+    reinterpret_cast<C*>(out.p[0])[o] = s0;
+    reinterpret_cast<C*>(out.p[1])[o] = s1;
+    reinterpret_cast<C*>(out.p[2])[o] = s2;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Pass 5: forward z transforms in fixed point, then the FP64 epilogue at each
-// thread's own positions.  Blocks, tiles and pruning are those of k_zfwd_epi.
+// thread's own positions.  Tiles and pruning are those of k_zfwd_epi.  TX: the
+// tile width; a quarter of the usual one (blocks of 64 threads) where the usual
+// tiles are fewer than two per SM, so that the epilogue's FP64 work spreads over
+// all SMs.
 // ---------------------------------------------------------------------------
-template <int LGZ>
-__global__ void __launch_bounds__(kFxTileThreads, 2)
+template <int LGZ, int TX>
+__global__ void __launch_bounds__(TX << (LGZ - 3), 512 / (TX << (LGZ - 3)))
 k_fx_zfwd(Ptr6 w, Ptr6 bc, Ptr6 out, DevTables<double> tb, Geom g, int mode, int pruned,
           const int32_t* __restrict__ tiles, FxExp ex, long long fxs, Batch<double> bt) {
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ unsigned slots[FxTileRed<LGZ>::kSlots];
-  constexpr int TX = fx_tile<LGZ>();
+  __shared__ unsigned slots[FxTileRed<TX>::kSlots];
   const int x = threadIdx.x % TX, t = threadIdx.x / TX;
   int tile = blockIdx.x, y = blockIdx.y;
   if (pruned) {
@@ -532,10 +605,11 @@ k_fx_zfwd(Ptr6 w, Ptr6 bc, Ptr6 out, DevTables<double> tb, Geom g, int mode, int
   constexpr int reg = strided_rows(1 << LGZ) * TX;
   const int4* tw = reinterpret_cast<const int4*>(tb.fwz);
   const long long xo = (long long)mem * fxs;
-  auto red = fx_red_tile<LGZ>(slots, x, t);
+  auto red = fx_red_tile<TX>(slots, x, t);
   red.clear_all();
   __syncthreads();
   E v[8];
+  int e[3];
 #pragma unroll 1
   for (int f = 0; f < 3; ++f) {
     E* S = reinterpret_cast<E*>(smraw) + f * reg;
@@ -549,16 +623,17 @@ k_fx_zfwd(Ptr6 w, Ptr6 bc, Ptr6 out, DevTables<double> tb, Geom g, int mode, int
       v[i] = E{shr_clamp(q.x, sh), shr_clamp(q.y, sh)};
     }
     const FxMem<LGZ, TX> mem_{S + x};
-    int e = top >= kFxNaN / 2 ? kFxNaN : top + (kFxOut - kFxIn);
-    e += fx_line<-1>(v, t, tw, mem_, BlockSync{}, red);
+    int ef = top >= kFxNaN / 2 ? kFxNaN : top + (kFxOut - kFxIn);
+    ef += fx_line<-1>(v, t, tw, mem_, BlockSync{}, red);
     red.par ^= 1;
-    mem_.own(t, [&](int i, E& o) {
-      reinterpret_cast<double2&>(o) = double2{fx_to_double(v[i].x, e), fx_to_double(v[i].y, e)};
-    });
+    mem_.own(t, [&](int i, E& o) { o = v[i]; });
+    if (f == 0) e[0] = ef;
+    if (f == 1) e[1] = ef;
+    if (f == 2) e[2] = ef;
   }
   if (!valid) return;   // no barrier follows
-  zfwd_epilogue<double, LGZ, 1>(reinterpret_cast<const double2*>(smraw), reg, StridedIdxLg{11 - LGZ, x}, t, X, y, ylim, base, plane, bc, out,
-                                tb, g, mode, pruned);
+  fx_epilogue<LGZ, TX>(reinterpret_cast<E*>(smraw) + x, reg, e, t, X, y, ylim, base, plane, bc, out, tb, g, mode,
+                       pruned);
 }
 
 }  // namespace gt

@@ -88,6 +88,7 @@ struct DevTables {
   const R* fkzs;   // [nz]
   const R* emk;    // by k2 (emk_by_k2) or [nz][ny][nh]
   int emk_by_k2;
+  const R* ik2;         // FP64 form, emk_by_k2: 1 / k2 by k2 (1 at 0)
   const int32_t* xcut;  // [nz][ny]
   const void* twx;      // twiddles exp(-2 pi i m / nx), m < nx  (complex R)
   const void* twy;      // ny

@@ -682,12 +682,16 @@ k_zk2(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, const int32
 // needs a third of the shared memory of k_zinv_curl and, with one or two
 // input fields live at a time, fewer registers: three resident blocks of 256
 // threads for FP32 instead of two.  Same columns, pruning and output, the
-// same expressions per element.
+// same expressions per element.  split: one output line per block (blockIdx.z =
+// 6 member + line in a full launch, line in a pruned one), for grids with
+// fewer tiles than SMs, where k_zinv_curl's chain of six transforms is the
+// pass's time (mixed, us: 64^3, 43 tiles, 15.6 -> 13.0; 128 x 128 x 32, 85 tiles,
+// 15.4 -> 12.4; but 128^3, 221 tiles, 18.9 -> 21.2).
 // ---------------------------------------------------------------------------
 template <typename R, int LGZ>
 __global__ void __launch_bounds__(kSpassThreads, sizeof(R) == 8 ? 2 : 3)
 k_zinv_curl1(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, const int32_t* __restrict__ tiles,
-             long long mstride) {
+             int split, long long mstride) {
   using C = Cplx<R>;
   constexpr int W = zcols<R>();
   using E = ColT<R, W>;
@@ -705,7 +709,8 @@ k_zinv_curl1(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, cons
   const bool valid = X0 < ylim;
   constexpr int T = 1 << (LGZ - 3);
   const size_t plane = (size_t)g.ny * g.nhp;
-  const size_t base = (size_t)y * g.nhp + (valid ? X0 : 0) + member_offset(mstride, pruned ? blockIdx.y : blockIdx.z);
+  const size_t base = (size_t)y * g.nhp + (valid ? X0 : 0) + member_offset(mstride, pruned ? blockIdx.y : (split ? blockIdx.z / 6 : blockIdx.z));
+  const int f0 = split ? (int)(blockIdx.z % 6) : 0, f1 = split ? f0 + 1 : 6;
   const StridedIdxLg idx{lgTP, xp};
   const C* tw = reinterpret_cast<const C*>(tb.twz);
   R kx[W], kxs[W];
@@ -718,7 +723,7 @@ k_zinv_curl1(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, cons
   const R ky = tb.fky[y], kys = tb.fkys[y];
   E v[8];
 #pragma unroll 1
-  for (int f = 0; f < 6; ++f) {
+  for (int f = f0; f < f1; ++f) {
     // the fields output f reads: u_0 <- (a1, a2), u_1 <- (a0, a2), u_2 <- (a0, a1); w_c <- a_c
     const C* p1 = reinterpret_cast<const C*>(a.at(f < 3 ? (f == 0 ? 1 : 0) : f - 3));
     const C* p2 = reinterpret_cast<const C*>(a.at(f == 2 ? 1 : 2));
@@ -2439,7 +2444,7 @@ static int set_smem_attrs() {
   es[n++] = allow_smem(k_fx_spass<2, LG>, optin); \
   es[n++] = allow_smem(k_fx_spass<3, LG>, optin); \
   es[n++] = allow_smem(k_fx_x<LG>, optin);        \
-  es[n++] = allow_smem(k_fx_zfwd<LG>, optin);
+  es[n++] = allow_smem(k_fx_zfwd<LG, fx_tile<LG>()>, optin);
   GT_ALLOW(3) GT_ALLOW(4) GT_ALLOW(5) GT_ALLOW(6) GT_ALLOW(7) GT_ALLOW(8) GT_ALLOW(9) GT_ALLOW(10)
 #undef GT_ALLOW
 #endif
@@ -2648,9 +2653,14 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
     pb.p[i] = bcor[i];
     po.p[i] = out[i];
   }
+  // fewer tiles than two per SM (grids up to 128^3): the six lines of the inverse pass on the grid,
+  // narrow tiles for the forward one (us, z inverse and forward: 64^3 42 -> 14 and 32 -> 23, 128^3 67 -> 44 and
+  // 52 -> 34)
+  const bool few = (size_t)zgrid.x * zgrid.y * zgrid.z < (size_t)2 * device_sms();
+  const dim3 zigrid(zgrid.x, zgrid.y, few ? (pruned ? 6 : 6 * nm) : zgrid.z);
   GT_HOOK(kKZinvCurl, true);
 #define GT_L(LG) \
-  k_fx_zinv<LG><<<zgrid, kFxTileThreads, zsmem, s>>>(pa, pw, tb, g, pruned, tb.ztl[lgt], ex, fxs, mstride);
+  k_fx_zinv<LG><<<zigrid, kFxTileThreads, zsmem, s>>>(pa, pw, tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
   GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   GT_HOOK(kKZinvCurl, false);
@@ -2674,10 +2684,21 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
   if ((rc = fx_spass<1>(g, w, 3, tb.fwy, s, hook, hctx, ex, xlim, pruned ? 2 : 0, tb.xcut, (int)nm, fxs, mstride)))
     return rc;
   GT_HOOK(kKZFwdEpi, true);
-#define GT_L(LG)                                                                                                  \
-  k_fx_zfwd<LG><<<zgrid, kFxTileThreads, 3 * zsmem, s>>>(pw, pb, po, tb, g, mode, pruned, tb.ztl[lgt], ex, fxs, bb);
-  GT_DISPATCH_LG(g.lnz, GT_L)
+  if (few && g.lnz <= 7) {
+    const int lgn = lgt - 2;
+    const dim3 ngrid = pruned ? dim3(tb.nztl[lgn], nm) : dim3((g.nh + (1 << lgn) - 1) >> lgn, g.ny, nm);
+#define GT_L(LG)                                                                                               \
+  k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4><<<ngrid, kFxTileThreads / 4, 3 * zsmem / 4, s>>>( \
+      pw, pb, po, tb, g, mode, pruned, tb.ztl[lgn], ex, fxs, bb);
+    GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
+  } else {
+#define GT_L(LG)                                                                                                \
+  k_fx_zfwd<LG, fx_tile<LG>()><<<zgrid, kFxTileThreads, 3 * zsmem, s>>>(pw, pb, po, tb, g, mode, pruned, tb.ztl[lgt], \
+                                                                        ex, fxs, bb);
+    GT_DISPATCH_LG(g.lnz, GT_L)
+#undef GT_L
+  }
   GT_HOOK(kKZFwdEpi, false);
   return (int)cudaGetLastError();
 }
@@ -2729,6 +2750,7 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
     for (int i = 0; i < 3; ++i) pa.p[i] = a[i];
     for (int i = 0; i < 6; ++i) pw.p[i] = w[i];
     const dim3 grid = pruned ? dim3(tb.nztl[c.lgTX], nm) : dim3(c.ntiles, g.ny, nm);
+    const bool few = (size_t)grid.x * grid.y * grid.z < (size_t)device_sms();
     GT_HOOK(kKZinvCurl, true);
     const bool fits = c.threads / zcols<R>() <= kSpassThreads;
     const int split = (ovl || (pm && pm->z_split == 1)) && fits ? 1 : 0;
@@ -2773,11 +2795,14 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
   }
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
-    } else if (pm && pm->z_split == 2 && fits) {
-      // one shared region, the input columns read again per output line
-#define GT_L(LG)                                                                                   \
-  k_zinv_curl1<R, LG><<<grid, c.threads / zcols<R>(), c.smem / 3, s>>>(pa, pw, tb, g, c.lgTX, pruned, \
-                                                                       tb.ztl[c.lgTX], mstride);
+    } else if (fits && !split && ((pm && pm->z_split == 2) || few)) {
+      // one shared region, the input columns read again per output line; where
+      // tiles are few, one line per block
+      const int fs = few && !(pm && pm->z_split == 2);
+      const dim3 gridf(grid.x, grid.y, fs ? (pruned ? 6 : 6 * nm) : grid.z);
+#define GT_L(LG)                                                                                    \
+  k_zinv_curl1<R, LG><<<gridf, c.threads / zcols<R>(), c.smem / 3, s>>>(pa, pw, tb, g, c.lgTX, pruned, \
+                                                                        tb.ztl[c.lgTX], fs, mstride);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
     } else {
@@ -2832,8 +2857,11 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
       // fit in xfused_threads and divide the number of row pairs
       const int T = gs.nx / 8;
       const long long npairs = (long long)gs.ny * gs.nz / 2;
+      // ... and, beyond a warp, leave two blocks per SM (16^3: one block of 256 threads 21 us, eight of 32 9 us)
+      const long long two = 2LL * device_sms();
       int P = 1;
-      while (P * 2 * T <= xfused_threads<R>() && npairs % (P * 2) == 0) P <<= 1;
+      while (P * 2 * T <= xfused_threads<R>() && npairs % (P * 2) == 0 && (P * T < 32 || npairs / (P * 2) * nm >= two))
+        P <<= 1;
       if (P * T > xfused_threads<R>() || npairs % P != 0) return (int)cudaErrorInvalidConfiguration;
       const int smem = P * gs.nx * csize;
       Ptr6 pw{};
