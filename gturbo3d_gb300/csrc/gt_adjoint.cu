@@ -9,6 +9,8 @@
 // invcurl, trunc and emk are self-adjoint, the Coriolis factor i omega kz has
 // adjoint -i omega kz, fft_dir^T = fft_inv / (NX NY NZ) and
 // fft_inv^T = (NX NY NZ) fft_dir.
+#include <algorithm>
+
 #include "gt_fft.cuh"
 #include "gt_internal.h"
 
@@ -20,162 +22,259 @@ struct P3 {
   void* p[3];
 };
 
-template <typename R>
-__device__ __forceinline__ void kvec(const DevTables<R>& tb, int X, int y, int z, R& kx, R& ky, R& kz) {
-  kx = tb.fkx[X];
-  ky = tb.fky[y];
-  kz = tb.fkz[z];
-}
-
-// out = op(a) (+ beta * b when accumulate), over all stored modes.
-//  op 0: curl a = i k x a                   op 1: k^2 a
-//  op 2: invcurl a (k = 0 left as is)       op 3: trunc (mask; k = 0 -> 0)
-//  op 4: i*sgn*omega*kz a                   op 5: emk a
-//  op 6: a (copy / axpy)                    op 7: 1{|k| >= kmin} a
-//  op 8: a with the k = 0 mode set to 0
-template <typename R>
-__global__ void k_spec_op(P3 out, P3 a, P3 b, DevTables<R> tb, Geom g, int op, R sgn, R kmin2, R beta,
-                          int accumulate) {
+// The step algebra's compound operators, one sweep each (a, b, c, o2 as named):
+//  kFuseTlTail   : o = trunc invcurl (a + i omega kz b)
+//  kFuseAdjHead  : o = invcurl trunc a, o2 += -i omega kz o
+//  kFuseAdjTail  : o = b + curl a + k^2 c
+//  kFuseStage    : o = Z E (a + f b)                     (Z: k = 0 mode to 0, E: emk)
+//  kFuseTlEnd    : o = Z E (E a + f b)
+//  kFuseAdjStart : o = f E Z a, o2 = E E Z a
+//  kFuseAdjMid   : t = E Z a, o2 += t, o = f t
+//  kFuseObj      : o = curl (1{|k| >= kmin} curl a)
+template <typename R, int OP>
+__global__ void __launch_bounds__(256)
+k_spec_fused(P3 out, P3 a, P3 b, P3 c, P3 o2, DevTables<R> tb, Geom g, R f, R kmin2) {
   using C = Cplx<R>;
   const size_t rows = (size_t)g.ny * g.nz;
-  for (size_t row = blockIdx.y; row < rows; row += gridDim.y) {
+  // a warp walks a row
+  const int lane = threadIdx.x & 31;
+  for (size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (size_t)gridDim.x * 8) {
     const int y = (int)(row % g.ny), z = (int)(row / g.ny);
-    for (int X = blockIdx.x * blockDim.x + threadIdx.x; X < g.nh; X += gridDim.x * blockDim.x) {
+    const R ky = tb.fky[y], kz = tb.fkz[z];
+    const int cut = tb.truncate ? tb.xcut[row] : g.nh;
+    for (int X = lane; X < g.nh; X += 32) {
       const size_t o = row * g.nhp + X;
-      C v[3];
-      for (int c = 0; c < 3; ++c) v[c] = reinterpret_cast<const C*>(a.p[c])[o];
-      R kx, ky, kz;
-      kvec(tb, X, y, z, kx, ky, kz);
+      auto ld = [&](const P3& p, C v[3]) {
+        for (int q = 0; q < 3; ++q) v[q] = reinterpret_cast<const C*>(p.p[q])[o];
+      };
+      auto st = [&](const P3& p, const C v[3]) {
+        for (int q = 0; q < 3; ++q) reinterpret_cast<C*>(p.p[q])[o] = v[q];
+      };
+      const R kx = tb.fkx[X];
       const R k2 = (tb.fkxs[X] + tb.fkys[y]) + tb.fkzs[z];
-      const bool zero_mode = (X == 0) && (y == 0) && (z == 0);
-      C r[3];
-      switch (op) {
-        case 0:
-          r[0] = C{-ky * v[2].y + kz * v[1].y, ky * v[2].x - kz * v[1].x};
-          r[1] = C{-kz * v[0].y + kx * v[2].y, kz * v[0].x - kx * v[2].x};
-          r[2] = C{-kx * v[1].y + ky * v[0].y, kx * v[1].x - ky * v[0].x};
-          break;
-        case 1:
-          for (int c = 0; c < 3; ++c) r[c] = C{k2 * v[c].x, k2 * v[c].y};
-          break;
-        case 2:
-          if (zero_mode) {
-            for (int c = 0; c < 3; ++c) r[c] = v[c];
-          } else {
-            const R qx = kx / k2, qy = ky / k2, qz = kz / k2;
-            r[0] = C{-qy * v[2].y + qz * v[1].y, qy * v[2].x - qz * v[1].x};
-            r[1] = C{-qz * v[0].y + qx * v[2].y, qz * v[0].x - qx * v[2].x};
-            r[2] = C{-qx * v[1].y + qy * v[0].y, qx * v[1].x - qy * v[0].x};
+      const bool zero_mode = X == 0 && row == 0;
+      const bool kill = tb.truncate && (zero_mode || X >= cut);
+      auto curl = [&](const C v[3], R sc, C r[3]) {   // i sc k x v
+        const R qx = sc * kx, qy = sc * ky, qz = sc * kz;
+        r[0] = C{-qy * v[2].y + qz * v[1].y, qy * v[2].x - qz * v[1].x};
+        r[1] = C{-qz * v[0].y + qx * v[2].y, qz * v[0].x - qx * v[2].x};
+        r[2] = C{-qx * v[1].y + qy * v[0].y, qx * v[1].x - qy * v[0].x};
+      };
+      C va[3], r[3];
+      if constexpr (OP == kFuseTlTail || OP == kFuseAdjHead) {
+        for (int q = 0; q < 3; ++q) r[q] = C{0, 0};
+        if (!kill) {
+          ld(a, va);
+          if constexpr (OP == kFuseTlTail) {
+            C vb[3];
+            ld(b, vb);
+            const R okz = tb.omega * kz;
+            for (int q = 0; q < 3; ++q) va[q] = C{va[q].x - okz * vb[q].y, va[q].y + okz * vb[q].x};
           }
-          break;
-        case 3: {
-          const bool kill = tb.truncate && (zero_mode || X >= tb.xcut[(size_t)z * g.ny + y]);
-          for (int c = 0; c < 3; ++c) r[c] = kill ? C{0, 0} : v[c];
-          break;
+          if (zero_mode) {
+            for (int q = 0; q < 3; ++q) r[q] = va[q];
+          } else {
+            curl(va, (R)1 / k2, r);
+          }
+          if constexpr (OP == kFuseAdjHead) {
+            C w[3];
+            ld(o2, w);
+            const R okz = tb.omega * kz;
+            for (int q = 0; q < 3; ++q) w[q] = C{w[q].x + okz * r[q].y, w[q].y - okz * r[q].x};
+            st(o2, w);
+          }
         }
-        case 4: {
-          const R f = sgn * tb.omega * kz;   // i f v = (-f v.y, f v.x)
-          for (int c = 0; c < 3; ++c) r[c] = C{-f * v[c].y, f * v[c].x};
-          break;
-        }
-        case 5: {
-          const R e = tb.emk_by_k2 ? tb.emk[(int)k2] : tb.emk[((size_t)z * g.ny + y) * g.nh + X];
-          for (int c = 0; c < 3; ++c) r[c] = C{e * v[c].x, e * v[c].y};
-          break;
-        }
-        case 7: {
-          const bool keep = k2 >= kmin2;
-          for (int c = 0; c < 3; ++c) r[c] = keep ? v[c] : C{0, 0};
-          break;
-        }
-        case 8:
-          for (int c = 0; c < 3; ++c) r[c] = zero_mode ? C{0, 0} : v[c];
-          break;
-        default:
-          for (int c = 0; c < 3; ++c) r[c] = v[c];
-      }
-      for (int c = 0; c < 3; ++c) {
-        C* po = reinterpret_cast<C*>(out.p[c]);
-        if (accumulate) {
-          const C w = reinterpret_cast<const C*>(b.p[c])[o];
-          po[o] = C{r[c].x + beta * w.x, r[c].y + beta * w.y};
+        st(out, r);
+      } else if constexpr (OP == kFuseAdjTail) {
+        C vb[3], vc[3];
+        ld(a, va);
+        ld(b, vb);
+        ld(c, vc);
+        curl(va, (R)1, r);
+        for (int q = 0; q < 3; ++q) r[q] = C{(vb[q].x + r[q].x) + k2 * vc[q].x, (vb[q].y + r[q].y) + k2 * vc[q].y};
+        st(out, r);
+      } else if constexpr (OP == kFuseObj) {
+        ld(a, va);
+        C u[3];
+        curl(va, (R)1, u);
+        if (!(k2 >= kmin2)) u[0] = u[1] = u[2] = C{0, 0};
+        curl(u, (R)1, r);
+        st(out, r);
+      } else {
+        const R e = tb.emk_by_k2 ? tb.emk[(int)k2] : tb.emk[row * g.nh + X];
+        ld(a, va);
+        if constexpr (OP == kFuseStage || OP == kFuseTlEnd) {
+          C vb[3];
+          ld(b, vb);
+          const R ea = OP == kFuseStage ? (R)1 : e;
+          for (int q = 0; q < 3; ++q)
+            r[q] = zero_mode ? C{0, 0} : C{e * (ea * va[q].x + f * vb[q].x), e * (ea * va[q].y + f * vb[q].y)};
+          st(out, r);
         } else {
-          po[o] = r[c];
+          C t[3], w[3];
+          for (int q = 0; q < 3; ++q) {
+            t[q] = zero_mode ? C{0, 0} : C{e * va[q].x, e * va[q].y};
+            r[q] = C{f * t[q].x, f * t[q].y};
+          }
+          if constexpr (OP == kFuseAdjStart) {
+            for (int q = 0; q < 3; ++q) w[q] = C{e * t[q].x, e * t[q].y};
+          } else {
+            ld(o2, w);
+            for (int q = 0; q < 3; ++q) w[q] = C{t[q].x + w[q].x, t[q].y + w[q].y};
+          }
+          st(o2, w);
+          st(out, r);
         }
       }
     }
   }
 }
 
-// out = s1 * (a x b) + s2 * (c x d) on real fields (d, c may be null).
-template <typename R>
-__global__ void k_phys_cross(P3 out, P3 a, P3 b, P3 c, P3 d, R s1, R s2, int two, size_t n) {
+template <typename R> __device__ __forceinline__ void cross3(const R a[3], const R b[3], R r[3]) {
+  r[0] = a[1] * b[2] - a[2] * b[1];
+  r[1] = a[2] * b[0] - a[0] * b[2];
+  r[2] = a[0] * b[1] - a[1] * b[0];
+}
+
+// Real fields.  ADJ false: o1 = c x b + a x d (du x w + u x dw for u, w, du, dw =
+// a, b, c, d).  ADJ true: o1 = b x c, o2 = c x a (w x g and g x u for g = c).
+template <typename R, bool ADJ>
+__global__ void k_phys_cross(P3 o1, P3 o2, P3 a, P3 b, P3 c, P3 d, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const R a0 = reinterpret_cast<const R*>(a.p[0])[i], a1 = reinterpret_cast<const R*>(a.p[1])[i],
-            a2 = reinterpret_cast<const R*>(a.p[2])[i];
-    const R b0 = reinterpret_cast<const R*>(b.p[0])[i], b1 = reinterpret_cast<const R*>(b.p[1])[i],
-            b2 = reinterpret_cast<const R*>(b.p[2])[i];
-    R r0 = s1 * (a1 * b2 - a2 * b1), r1 = s1 * (a2 * b0 - a0 * b2), r2 = s1 * (a0 * b1 - a1 * b0);
-    if (two) {
-      const R c0 = reinterpret_cast<const R*>(c.p[0])[i], c1 = reinterpret_cast<const R*>(c.p[1])[i],
-              c2 = reinterpret_cast<const R*>(c.p[2])[i];
-      const R d0 = reinterpret_cast<const R*>(d.p[0])[i], d1 = reinterpret_cast<const R*>(d.p[1])[i],
-              d2 = reinterpret_cast<const R*>(d.p[2])[i];
-      r0 += s2 * (c1 * d2 - c2 * d1);
-      r1 += s2 * (c2 * d0 - c0 * d2);
-      r2 += s2 * (c0 * d1 - c1 * d0);
+    R u[3], w[3], x[3], y[3], r[3], q[3];
+    for (int k = 0; k < 3; ++k) {
+      u[k] = reinterpret_cast<const R*>(a.p[k])[i];
+      w[k] = reinterpret_cast<const R*>(b.p[k])[i];
+      x[k] = reinterpret_cast<const R*>(c.p[k])[i];
+      if (!ADJ) y[k] = reinterpret_cast<const R*>(d.p[k])[i];
     }
-    reinterpret_cast<R*>(out.p[0])[i] = r0;
-    reinterpret_cast<R*>(out.p[1])[i] = r1;
-    reinterpret_cast<R*>(out.p[2])[i] = r2;
+    if constexpr (ADJ) {
+      cross3(w, x, r);
+      cross3(x, u, q);
+    } else {
+      cross3(x, w, r);
+      cross3(u, y, q);
+    }
+    for (int k = 0; k < 3; ++k) {
+      if constexpr (ADJ) {
+        reinterpret_cast<R*>(o1.p[k])[i] = r[k];
+        reinterpret_cast<R*>(o2.p[k])[i] = q[k];
+      } else {
+        reinterpret_cast<R*>(o1.p[k])[i] = r[k] + q[k];
+      }
+    }
   }
+}
+
+// partial[block] = the block's part of sum over modes with k2 >= kmin2 of
+// fac |(curl b)|^2, products and sums in FP64; k_shell_sum adds them in order.
+constexpr int kShellThreads = 256;
+template <typename R>
+__global__ void __launch_bounds__(kShellThreads)
+k_shell_energy(P3 b, DevTables<R> tb, Geom g, R kmin2, double* partial) {
+  using C = Cplx<R>;
+  const size_t rows = (size_t)g.ny * g.nz;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double acc = 0.0;
+  for (size_t row = (size_t)blockIdx.x * 8 + warp; row < rows; row += (size_t)gridDim.x * 8) {
+    const int y = (int)(row % g.ny), z = (int)(row / g.ny);
+    const R ky = tb.fky[y], kz = tb.fkz[z];
+    for (int X = lane; X < g.nh; X += 32) {
+      const R kx = tb.fkx[X];
+      const R k2 = (tb.fkxs[X] + tb.fkys[y]) + tb.fkzs[z];
+      if (!(k2 >= kmin2)) continue;
+      const size_t o = row * g.nhp + X;
+      const C v0 = reinterpret_cast<const C*>(b.p[0])[o], v1 = reinterpret_cast<const C*>(b.p[1])[o],
+              v2 = reinterpret_cast<const C*>(b.p[2])[o];
+      const double r0 = -ky * v2.y + kz * v1.y, i0 = ky * v2.x - kz * v1.x;
+      const double r1 = -kz * v0.y + kx * v2.y, i1 = kz * v0.x - kx * v2.x;
+      const double r2 = -kx * v1.y + ky * v0.y, i2 = kx * v1.x - ky * v0.x;
+      const double fac = (X == 0 || X == g.nh - 1) ? 0.5 : 1.0;
+      acc += fac * (((r0 * r0 + i0 * i0) + (r1 * r1 + i1 * i1)) + (r2 * r2 + i2 * i2));
+    }
+  }
+  __shared__ double red[kShellThreads / 32];
+  for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+  if (lane == 0) red[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < kShellThreads / 32; ++w) s += red[w];
+    partial[blockIdx.x] = s;
+  }
+}
+__global__ void __launch_bounds__(256) k_shell_sum(double* partial, int n, double* out) {
+  __shared__ double red[256];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += 256) s += partial[i];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int h = 128; h > 0; h >>= 1) {
+    if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *out = red[0];
+}
+
+P3 p3(void* const p[3], void* const fallback[3]) {
+  P3 r;
+  for (int c = 0; c < 3; ++c) r.p[c] = (p ? p : fallback)[c];
+  return r;
 }
 
 }  // namespace
 
 template <typename R>
-int launch_spec_op(const Geom& g, const DevTables<R>& tb, void* const out[3], void* const a[3],
-                   void* const b[3], int op, double sgn, double kmin2, double beta, void* stream) {
-  P3 po{}, pa{}, pb{};
-  for (int c = 0; c < 3; ++c) {
-    po.p[c] = out[c];
-    pa.p[c] = a[c];
-    pb.p[c] = b ? b[c] : a[c];
+int launch_spec_fused(const Geom& g, const DevTables<R>& tb, int op, void* const out[3], void* const a[3],
+                      void* const b[3], void* const c[3], void* const o2[3], double f, double kmin2, void* stream) {
+  const size_t rows = (size_t)g.ny * g.nz;
+  const int blocks = (int)std::min<size_t>((rows + 7) / 8, 152 * 16);
+  const P3 po = p3(out, out), pa = p3(a, a), pb = p3(b, a), pc = p3(c, a), p2 = p3(o2, out);
+  switch (op) {
+#define GT_OP(OP)                                                                                          \
+  case OP:                                                                                                 \
+    k_spec_fused<R, OP><<<blocks, 256, 0, (cudaStream_t)stream>>>(po, pa, pb, pc, p2, tb, g, (R)f, (R)kmin2); \
+    break;
+    GT_OP(kFuseTlTail) GT_OP(kFuseAdjHead) GT_OP(kFuseAdjTail) GT_OP(kFuseStage) GT_OP(kFuseTlEnd)
+    GT_OP(kFuseAdjStart) GT_OP(kFuseAdjMid) GT_OP(kFuseObj)
+#undef GT_OP
+    default: return (int)cudaErrorInvalidValue;
   }
-  const int threads = 128;
-  const int bx = (g.nh + threads - 1) / threads;
-  const int by = (int)std::min<long long>((long long)g.ny * g.nz, 65535);
-  k_spec_op<R><<<dim3(bx, by), threads, 0, (cudaStream_t)stream>>>(po, pa, pb, tb, g, op, (R)sgn, (R)kmin2,
-                                                                    (R)beta, b ? 1 : 0);
   return (int)cudaGetLastError();
 }
 
 template <typename R>
-int launch_phys_cross(const Geom& g, void* const out[3], void* const a[3], void* const b[3],
-                      void* const c[3], void* const d[3], double s1, double s2, void* stream) {
-  P3 po{}, pa{}, pb{}, pc{}, pd{};
-  for (int i = 0; i < 3; ++i) {
-    po.p[i] = out[i];
-    pa.p[i] = a[i];
-    pb.p[i] = b[i];
-    pc.p[i] = c ? c[i] : a[i];
-    pd.p[i] = d ? d[i] : b[i];
-  }
+int launch_phys_cross(const Geom& g, int adjoint, void* const o1[3], void* const o2[3], void* const a[3],
+                      void* const b[3], void* const c[3], void* const d[3], void* stream) {
   const size_t n = (size_t)g.nx * g.ny * g.nz;
   const int threads = 256;
   const int blocks = (int)std::min<size_t>((n + threads - 1) / threads, 152 * 16);
-  k_phys_cross<R><<<blocks, threads, 0, (cudaStream_t)stream>>>(po, pa, pb, pc, pd, (R)s1, (R)s2,
-                                                                 c != nullptr, n);
+  const P3 po = p3(o1, o1), p2 = p3(o2, o1), pa = p3(a, a), pb = p3(b, a), pc = p3(c, a), pd = p3(d, a);
+  if (adjoint)
+    k_phys_cross<R, true><<<blocks, threads, 0, (cudaStream_t)stream>>>(po, p2, pa, pb, pc, pd, n);
+  else
+    k_phys_cross<R, false><<<blocks, threads, 0, (cudaStream_t)stream>>>(po, p2, pa, pb, pc, pd, n);
   return (int)cudaGetLastError();
 }
 
-template int launch_spec_op<float>(const Geom&, const DevTables<float>&, void* const*, void* const*,
-                                   void* const*, int, double, double, double, void*);
-template int launch_spec_op<double>(const Geom&, const DevTables<double>&, void* const*, void* const*,
-                                    void* const*, int, double, double, double, void*);
-template int launch_phys_cross<float>(const Geom&, void* const*, void* const*, void* const*, void* const*,
-                                      void* const*, double, double, void*);
-template int launch_phys_cross<double>(const Geom&, void* const*, void* const*, void* const*, void* const*,
-                                       void* const*, double, double, void*);
+template <typename R>
+int launch_shell_energy(const Geom& g, const DevTables<R>& tb, void* const b[3], double kmin2, double* partials,
+                        int cap, double* result, void* stream) {
+  const size_t rows = (size_t)g.ny * g.nz;
+  const int blocks = (int)std::min<size_t>((rows + 7) / 8, (size_t)std::min(cap, 152 * 8));
+  k_shell_energy<R><<<blocks, kShellThreads, 0, (cudaStream_t)stream>>>(p3(b, b), tb, g, (R)kmin2, partials);
+  k_shell_sum<<<1, 256, 0, (cudaStream_t)stream>>>(partials, blocks, result);
+  return (int)cudaGetLastError();
+}
+
+#define GT_INST_ADJ(R)                                                                                             \
+  template int launch_spec_fused<R>(const Geom&, const DevTables<R>&, int, void* const*, void* const*, void* const*, \
+                                    void* const*, void* const*, double, double, void*);                            \
+  template int launch_phys_cross<R>(const Geom&, int, void* const*, void* const*, void* const*, void* const*,      \
+                                    void* const*, void* const*, void*);                                            \
+  template int launch_shell_energy<R>(const Geom&, const DevTables<R>&, void* const*, double, double*, int, double*, \
+                                      void*);
+GT_INST_ADJ(float)
+GT_INST_ADJ(double)
 
 }  // namespace gt

@@ -269,6 +269,7 @@ void free_handle(gt_handle* h) {
   }
   if (h->sg.exec) cudaGraphExecDestroy(h->sg.exec);
   if (h->d_force) cudaFree(h->d_force);
+  if (h->adj_mem) cudaFree(h->adj_mem);
   if (h->fields_mem && h->owns_fields) cudaFree(h->fields_mem);
   if (h->stage) cudaFree(h->stage);
   if (h->tab_mem) cudaFree(h->tab_mem);
@@ -395,14 +396,14 @@ int download_real(gt_handle* h, const void* src, double* host) {
   return GT_OK;
 }
 
-int fft_inv_dev(gt_handle* h, void* spec, void* real) {
-  if (h->mixed) return launch_fft_inv<float>(h->g, h->t32, spec, real, h->w, h->stream, hook_fn, h);
-  return launch_fft_inv<double>(h->g, h->t64, spec, real, h->w, h->stream, hook_fn, h);
+int fft_inv_dev(gt_handle* h, void* const* spec, void* const* real, int nf, int pruned) {
+  if (h->mixed) return launch_fft_inv<float>(h->g, h->t32, spec, real, nf, pruned, &h->pm, h->stream, hook_fn, h);
+  return launch_fft_inv<double>(h->g, h->t64, spec, real, nf, pruned, &h->pm, h->stream, hook_fn, h);
 }
 
-int fft_dir_dev(gt_handle* h, const void* real, void* spec) {
-  if (h->mixed) return launch_fft_dir<float>(h->g, h->t32, real, spec, h->w, h->stream, hook_fn, h);
-  return launch_fft_dir<double>(h->g, h->t64, real, spec, h->w, h->stream, hook_fn, h);
+int fft_dir_dev(gt_handle* h, void* const* real, void* const* spec, int nf) {
+  if (h->mixed) return launch_fft_dir<float>(h->g, h->t32, real, spec, nf, &h->pm, h->stream, hook_fn, h);
+  return launch_fft_dir<double>(h->g, h->t64, real, spec, nf, &h->pm, h->stream, hook_fn, h);
 }
 
 int point(gt_handle* h, void* const a[3], int op, double* partial, int npartial) {
@@ -860,7 +861,7 @@ int gt_fft_dir(gt_handle* h, const double* real_in, double* spec_out) {
   int rc = set_dev(h);
   if (rc) return rc;
   if ((rc = upload_real(h, real_in, h->w[1]))) return rc;
-  CKI(fft_dir_dev(h, h->w[1], h->w[0]));
+  CKI(fft_dir_dev(h, h->w + 1, h->w, 1));
   prefault(&spec_out, 1, spec_bytes(h->g));
   if ((rc = download_spec(h, h->w[0], spec_out))) return rc;
   CK(cudaStreamSynchronize(h->stream));
@@ -872,7 +873,7 @@ int gt_fft_inv(gt_handle* h, const double* spec_in, double* real_out) {
   int rc = set_dev(h);
   if (rc) return rc;
   if ((rc = upload_spec(h, spec_in, h->w[0]))) return rc;
-  CKI(fft_inv_dev(h, h->w[0], h->w[1]));
+  CKI(fft_inv_dev(h, h->w, h->w + 1, 1, 0));
   prefault(&real_out, 1, real_bytes(h->g));
   if ((rc = download_real(h, h->w[1], real_out))) return rc;
   CK(cudaStreamSynchronize(h->stream));
@@ -886,11 +887,11 @@ int gt_velocity(gt_handle* h, double* ux, double* uy, double* uz) {
   void* const u[3] = {h->w[3], h->w[4], h->w[5]};
   if ((rc = copy_fields(h, u, h->b))) return rc;
   CKI(point(h, u, 0, nullptr, 0));                        // curl (main.f90:195)
+  CKI(fft_inv_dev(h, u, h->w, 3, use_pruning(h) ? 1 : 0));   // fft_inv x3 (main.f90:197-199)
   double* dst[3] = {ux, uy, uz};
   prefault(dst, 3, real_bytes(h->g));
-  for (int c = 0; c < 3; ++c) {                           // fft_inv x3 (main.f90:197-199)
-    CKI(fft_inv_dev(h, u[c], h->w[0]));
-    if ((rc = download_real(h, h->w[0], dst[c]))) return rc;
+  for (int c = 0; c < 3; ++c) {
+    if ((rc = download_real(h, h->w[c], dst[c]))) return rc;
     CK(cudaStreamSynchronize(h->stream));
   }
   return GT_OK;
@@ -903,11 +904,9 @@ int gt_set_state_physical(gt_handle* h, const double* ux, const double* uy, cons
   if (rc) return rc;
   void* const a[3] = {h->w[3], h->w[4], h->w[5]};
   const double* src[3] = {ux, uy, uz};
-  for (int c = 0; c < 3; ++c) {                           // fft_dir x3 (main.f90:91-93)
-    if ((rc = upload_real(h, src[c], h->w[0]))) return rc;
-    CKI(fft_dir_dev(h, h->w[0], a[c]));
-    CK(cudaStreamSynchronize(h->stream));                 // staging reuse
-  }
+  for (int c = 0; c < 3; ++c)
+    if ((rc = upload_real(h, src[c], h->w[c]))) return rc;
+  CKI(fft_dir_dev(h, h->w, a, 3));                        // fft_dir x3 (main.f90:91-93)
   CKI(point(h, a, 3, h->d_partials, h->npartials));       // incompr (main.f90:96)
   CKI(point(h, a, 1, nullptr, 0));                        // invcurl (main.f90:99)
   if (h->p.truncate == 1) CKI(point(h, a, 2, nullptr, 0));  // trunc x3 (main.f90:102-106)

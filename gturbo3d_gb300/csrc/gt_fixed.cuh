@@ -282,23 +282,24 @@ template <int LGL, typename Red> __device__ __forceinline__ unsigned fx_top_get(
 __device__ __forceinline__ int fx_headroom(unsigned top) { return max(0, __clz((int)top) - (64 - kFxOut)); }
 
 // ---- exponents of the fixed-point work fields -----------------------------
-// One int per line beside the work fields, in scratch the FP64 handle owns
-// anyway (its transfer staging field); all members' scratch mstride ints apart.
+// One int per line beside up to six work fields, in scratch the FP64 handle owns
+// anyway (its transfer staging field, 4 nz ny nhp ints, which holds them for every
+// grid of 8 points and more an axis).
 struct FxExp {
   int* ez;    // [6][ny][nhp]  lines along z (inverse), by column (x, y)
   int* ey;    // [6][nz][nhp]  lines along y (inverse)
-  int* ex;    // [3][nz][ny]   lines along x (forward)
-  int* eyf;   // [3][nz][nhp]  lines along y (forward)
+  int* ex;    // [6][nz][ny]   lines along x (forward)
+  int* eyf;   // [6][nz][nhp]  lines along y (forward)
   int* mz;    // [6][nhp]      max of ez over y
   int* my;    // [6][nz]       max of ey over x
-  int* mx;    // [3][nz]       max of ex over y
-  int* myf;   // [3][nhp]      max of eyf over z
+  int* mx;    // [6][nz]       max of ex over y
+  int* myf;   // [6][nhp]      max of eyf over z
   size_t max_bytes;   // mz..myf, contiguous, set to kFxUnsetByte before the passes run
 };
 constexpr int kFxUnsetByte = 0x80;   // ints of -2139062144, below every exponent
 
 static inline size_t fx_exp_ints(int ny, int nz, int nhp) {
-  return (size_t)9 * nhp + (size_t)9 * nz + (size_t)6 * ny * nhp + (size_t)9 * nz * nhp + (size_t)3 * nz * ny;
+  return (size_t)12 * nhp + (size_t)12 * nz + (size_t)6 * ny * nhp + (size_t)12 * nz * nhp + (size_t)6 * nz * ny;
 }
 static inline FxExp fx_exp(void* scratch, int ny, int nz, int nhp) {
   FxExp e;
@@ -306,13 +307,13 @@ static inline FxExp fx_exp(void* scratch, int ny, int nz, int nhp) {
   auto take = [&](size_t n) { int* r = p; p += n; return r; };
   e.mz = take((size_t)6 * nhp);
   e.my = take((size_t)6 * nz);
-  e.mx = take((size_t)3 * nz);
-  e.myf = take((size_t)3 * nhp);
-  e.max_bytes = ((size_t)9 * nhp + 9 * (size_t)nz) * sizeof(int);
+  e.mx = take((size_t)6 * nz);
+  e.myf = take((size_t)6 * nhp);
+  e.max_bytes = ((size_t)12 * nhp + 12 * (size_t)nz) * sizeof(int);
   e.ez = take((size_t)6 * ny * nhp);
   e.ey = take((size_t)6 * nz * nhp);
-  e.ex = take((size_t)3 * nz * ny);
-  e.eyf = take((size_t)3 * nz * nhp);
+  e.ex = take((size_t)6 * nz * ny);
+  e.eyf = take((size_t)6 * nz * nhp);
   return e;
 }
 

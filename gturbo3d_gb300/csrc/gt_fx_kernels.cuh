@@ -141,9 +141,13 @@ k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim
   __shared__ int emax[KIND == 2 ? kFxLines : 1];
   const int x = threadIdx.x % TX, t = threadIdx.x / TX;
   const int X = blockIdx.x * TX + x;
+  const int fi = blockIdx.z % nf, mem = blockIdx.z / nf, o = blockIdx.y;
+  if (KIND == 2 && ymask == 3) {   // kept columns: X < xcut0[y]
+    xlim = min(xlim, xcut0[o]);
+    if ((int)blockIdx.x * TX >= xlim) return;
+  }
   const bool valid = X < xlim;
   constexpr int T = 1 << (LGL - 3);
-  const int fi = blockIdx.z % nf, mem = blockIdx.z / nf, o = blockIdx.y;
   E* p = reinterpret_cast<E*>(f.at(fi));
   const size_t base = (size_t)o * (size_t)os + (valid ? X : 0) + member_offset(mstride, mem);
   auto red = fx_red_tile<TX>(slots, x, t);
@@ -427,22 +431,24 @@ k_fx_x(Ptr6 w, Geom g, const void* twv, int xa, int lgscale, FxExp ex, long long
 // Plain x transforms of one field (rows packed in pairs).
 template <int LGN>
 __global__ void __launch_bounds__(256)
-k_fx_xc2r(const void* specv, double* __restrict__ real, Geom g, const void* twv, int P, FxExp ex) {
+k_fx_xc2r(Ptr6 specs, Ptr6 reals, Geom g, const void* twv, int P, int xa, FxExp ex) {
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ unsigned slots[FxRowRed<LGN, 1>::kSlots];
   constexpr int N = 1 << LGN, lgT = LGN - 3, T = 1 << lgT, LN = FxMem<LGN, 1>::kRows;
   const int p = threadIdx.x >> lgT, t = threadIdx.x & (T - 1);
   const size_t pair = (size_t)blockIdx.x * P + p;
-  const E* X1 = reinterpret_cast<const E*>(specv) + (2 * pair) * g.nhp;
+  const int f = blockIdx.y;   // field
+  const E* X1 = reinterpret_cast<const E*>(specs.at(f)) + (2 * pair) * g.nhp;
   const E* X2 = X1 + g.nhp;
+  double* real = reinterpret_cast<double*>(reals.at(f));
   const int z = (int)((2 * pair) >> g.lny);
-  const int* e1 = ex.ey + (size_t)z * g.nhp;   // both rows lie in plane z
-  const int top = ex.my[z];
+  const int* e1 = ex.ey + ((size_t)f * g.nz + z) * g.nhp;   // both rows lie in plane z
+  const int top = ex.my[(size_t)f * g.nz + z];
   auto red = fx_red_rows<LGN, 1>(slots, p, t);
   red.clear_all();
   E v[8];
-  for8([&](auto I) { v[I] = fx_pack_c2r<I, N>(X1, X2, e1, e1, top, t, g.nh); });
+  for8([&](auto I) { v[I] = fx_pack_c2r<I, N>(X1, X2, e1, e1, top, t, xa); });
   int e = top >= kFxNaN / 2 ? kFxNaN : top + (kFxOut - kFxIn + 1);
   __syncthreads();
   const FxMem<LGN, 1> mem{reinterpret_cast<E*>(smraw) + p * LN};
@@ -458,7 +464,7 @@ k_fx_xc2r(const void* specv, double* __restrict__ real, Geom g, const void* twv,
 
 template <int LGN>
 __global__ void __launch_bounds__(256)
-k_fx_xr2c(const double* __restrict__ real, void* specv, Geom g, const void* twv, int P, int lgscale, FxExp ex) {
+k_fx_xr2c(Ptr6 reals, Ptr6 specs, Geom g, const void* twv, int P, int lgscale, FxExp ex) {
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ unsigned slots[FxRowRed<LGN, 1>::kSlots];
@@ -466,7 +472,8 @@ k_fx_xr2c(const double* __restrict__ real, void* specv, Geom g, const void* twv,
   constexpr int N = 1 << LGN, lgT = LGN - 3, T = 1 << lgT, LN = FxMem<LGN, 1>::kRows;
   const int p = threadIdx.x >> lgT, t = threadIdx.x & (T - 1);
   const size_t pair = (size_t)blockIdx.x * P + p;
-  const double* r0 = real + (2 * pair) * (size_t)N;
+  const int f = blockIdx.y;   // field
+  const double* r0 = reinterpret_cast<const double*>(reals.at(f)) + (2 * pair) * (size_t)N;
   const double* r1 = r0 + N;
   auto red = fx_red_rows<LGN, 1>(slots, p, t);
   red.clear_all();
@@ -495,13 +502,14 @@ k_fx_xr2c(const double* __restrict__ real, void* specv, Geom g, const void* twv,
   const unsigned mag = fx_top_put<LGN>(red, fx_or_hi(v), 0);
   __syncthreads();
   const int u = fx_headroom(fx_top_get<LGN>(red, mag, 0));
-  E* spec = reinterpret_cast<E*>(specv);
+  E* spec = reinterpret_cast<E*>(specs.at(f));
   fx_split<false>(mem, t, g.nh, u, spec + (2 * pair) * (size_t)g.nhp, spec + (2 * pair + 1) * (size_t)g.nhp);
   if (t == 0) {
     if (e < kFxNaN / 2) e -= u + lgscale;
-    ex.ex[2 * pair] = e;
-    ex.ex[2 * pair + 1] = e;
-    atomicMax(&ex.mx[(int)((2 * pair) >> g.lny)], e);
+    int* eo = ex.ex + (size_t)f * g.nz * g.ny + 2 * pair;
+    eo[0] = e;
+    eo[1] = e;
+    atomicMax(&ex.mx[(size_t)f * g.nz + ((2 * pair) >> g.lny)], e);
   }
 }
 

@@ -68,6 +68,10 @@ struct gt_handle {
     int64_t steps = 0;           // steps taken with this key
     bool broken = false;         // capture or instantiation failed once
   } sg;
+  // workspace of the tangent-linear, adjoint and gradient calls, kept with the
+  // handle up to a bound (gt_tl_adj.cu)
+  void* adj_mem = nullptr;
+  size_t adj_bytes = 0;
   double* d_partials = nullptr;
   int npartials = 0;
   double* d_result = nullptr;

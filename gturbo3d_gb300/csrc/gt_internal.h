@@ -228,13 +228,19 @@ int launch_convert(const Geom& g, const void* src, void* dst, int to_working, vo
 template <typename R>
 int launch_pack_rows(const Geom& g, void* packed, void* field, int to_working, void* stream, LaunchHook hook,
                      void* hctx);
-// Plain 3D transforms of one field (real layout [nz][ny][nx] in w-buffers).
+// Plain 3D transforms of nf <= 6 fields (real layout [nz][ny][nx]); pm supplies
+// the FP64 form's scratch.
 template <typename R>
-int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* spec, void* real_out,
-                   void* const w[6], void* stream, LaunchHook hook, void* hctx);
+int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* const* spec, void* const* real, int nf, int pruned,
+                   const PassTuning* pm, void* stream, LaunchHook hook, void* hctx);
 template <typename R>
-int launch_fft_dir(const Geom& g, const DevTables<R>& tb, const void* real_in, void* spec_out,
-                   void* const w[6], void* stream, LaunchHook hook, void* hctx);
+int launch_fft_dir(const Geom& g, const DevTables<R>& tb, void* const* real, void* const* spec, int nf,
+                   const PassTuning* pm, void* stream, LaunchHook hook, void* hctx);
+// u = curl a and w = k^2 a in physical space (w6: six spectral work fields).
+template <typename R>
+int launch_phys_uw(const Geom& g, const DevTables<R>& tb, void* const a[3], void* const w6[6], void* const u[3],
+                   void* const w[3], int pruned, const PassTuning* pm, int* err, void* stream, LaunchHook hook,
+                   void* hctx);
 // Pointwise spectral ops used by the output and initial-state paths.
 // op: 0 = curl, 1 = invcurl, 2 = trunc, 3 = incompr (writes |k.a|^2 partials)
 template <typename R>
@@ -252,12 +258,17 @@ template <typename R>
 int launch_energy(const Geom& g, const DevTables<R>& tb, void* const b[3], int pruned, double* partials,
                   int nblocks, double* result, void* stream, LaunchHook hook, void* hctx);
 int diag_blocks(const Geom& g);
-// Tangent-linear / adjoint building blocks (gt_adjoint.cu): out = op(a) [+ beta b].
+// Tangent-linear / adjoint building blocks (gt_adjoint.cu, where the operators are defined).
+enum FusedOp { kFuseTlTail, kFuseAdjHead, kFuseAdjTail, kFuseStage, kFuseTlEnd, kFuseAdjStart, kFuseAdjMid, kFuseObj };
 template <typename R>
-int launch_spec_op(const Geom& g, const DevTables<R>& tb, void* const out[3], void* const a[3],
-                   void* const b[3], int op, double sgn, double kmin2, double beta, void* stream);
+int launch_spec_fused(const Geom& g, const DevTables<R>& tb, int op, void* const out[3], void* const a[3],
+                      void* const b[3], void* const c[3], void* const o2[3], double f, double kmin2, void* stream);
 template <typename R>
-int launch_phys_cross(const Geom& g, void* const out[3], void* const a[3], void* const b[3],
-                      void* const c[3], void* const d[3], double s1, double s2, void* stream);
+int launch_phys_cross(const Geom& g, int adjoint, void* const o1[3], void* const o2[3], void* const a[3],
+                      void* const b[3], void* const c[3], void* const d[3], void* stream);
+// J of gt_objective for the spectral fields b.
+template <typename R>
+int launch_shell_energy(const Geom& g, const DevTables<R>& tb, void* const b[3], double kmin2, double* partials,
+                        int cap, double* result, void* stream);
 
 }  // namespace gt

@@ -787,6 +787,10 @@ k_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTX, i
   const int TX = 1 << lgTX;
   const int x = threadIdx.x & (TX - 1), t = threadIdx.x >> lgTX;
   const int X = blockIdx.x * TX + x;
+  if (ymask == 3) {   // z pass over kept columns: X < xcut0[y]
+    xlim = min(xlim, xcut0[blockIdx.y]);
+    if ((int)blockIdx.x * TX >= xlim) return;
+  }
   const bool valid = X < xlim;
   constexpr int T = 1 << (LGL - 3);
   // blockIdx.z = member * nf + field
@@ -834,6 +838,10 @@ k_spass2(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTP, 
   const int TP = 1 << lgTP;
   const int xp = threadIdx.x & (TP - 1), t = threadIdx.x >> lgTP;
   const int X0 = 2 * (blockIdx.x * TP + xp);
+  if (ymask == 3) {   // z pass over kept columns: X < xcut0[y]
+    xlim = min(xlim, xcut0[blockIdx.y]);
+    if (2 * (int)blockIdx.x * TP >= xlim) return;
+  }
   constexpr int T = 1 << (LGL - 3);
   // blockIdx.z = member * nf + field
   C* p = reinterpret_cast<C*>(f.at(blockIdx.z % nf));
@@ -1835,7 +1843,7 @@ k_zfwd_zinv(Ptr6 w, Ptr6 bc, DevTables<R> tb, Geom g, int lgTX, int pruned, cons
 // ---------------------------------------------------------------------------
 template <typename R, int LGN>
 __global__ void __launch_bounds__(max_threads<R>())
-k_xc2r(const void* specv, R* __restrict__ real, Geom g, const void* twv, int P) {
+k_xc2r(Ptr6 specs, Ptr6 reals, Geom g, const void* twv, int P, int xa) {
   using C = Cplx<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
@@ -1843,12 +1851,13 @@ k_xc2r(const void* specv, R* __restrict__ real, Geom g, const void* twv, int P) 
   constexpr int LP = N;
   const int p = threadIdx.x >> lgT, t = threadIdx.x & (T - 1);
   const size_t pair = (size_t)blockIdx.x * P + p;
-  const C* spec = reinterpret_cast<const C*>(specv);
+  const C* spec = reinterpret_cast<const C*>(specs.at(blockIdx.y));   // field blockIdx.y
+  R* real = reinterpret_cast<R*>(reals.at(blockIdx.y));
   const C* X1 = spec + (2 * pair) * g.nhp;
   const C* X2 = spec + (2 * pair + 1) * g.nhp;
   C v[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = pack_c2r<R>(X1, X2, t + i * T, N, g.nh);
+  for (int i = 0; i < 8; ++i) v[i] = pack_c2r<R>(X1, X2, t + i * T, N, xa);
   fft_line_ct<+1, R, LGN>(v, t, reinterpret_cast<const C*>(twv), sm, SwzIdx{p * LP});
   R* r0 = real + (2 * pair) * (size_t)N;
   R* r1 = real + (2 * pair + 1) * (size_t)N;
@@ -1861,7 +1870,7 @@ k_xc2r(const void* specv, R* __restrict__ real, Geom g, const void* twv, int P) 
 
 template <typename R, int LGN>
 __global__ void __launch_bounds__(max_threads<R>())
-k_xr2c(const R* __restrict__ real, void* specv, Geom g, const void* twv, int P, R shalf) {
+k_xr2c(Ptr6 reals, Ptr6 specs, Geom g, const void* twv, int P, R shalf) {
   using C = Cplx<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
@@ -1869,6 +1878,7 @@ k_xr2c(const R* __restrict__ real, void* specv, Geom g, const void* twv, int P, 
   constexpr int LP = N;
   const int p = threadIdx.x >> lgT, t = threadIdx.x & (T - 1);
   const size_t pair = (size_t)blockIdx.x * P + p;
+  const R* real = reinterpret_cast<const R*>(reals.at(blockIdx.y));   // field blockIdx.y
   const R* r0 = real + (2 * pair) * (size_t)N;
   const R* r1 = real + (2 * pair + 1) * (size_t)N;
   C v[8];
@@ -1879,7 +1889,7 @@ k_xr2c(const R* __restrict__ real, void* specv, Geom g, const void* twv, int P, 
 #pragma unroll
   for (int i = 0; i < 8; ++i) sm[idx(t + i * T)] = v[i];
   __syncthreads();
-  C* spec = reinterpret_cast<C*>(specv);
+  C* spec = reinterpret_cast<C*>(specs.at(blockIdx.y));
   const int nh = g.nh;
   for (int n = threadIdx.x; n < P * 2 * nh; n += blockDim.x) {
     const int k = n % nh, rest = n / nh, r = rest & 1, pp = rest >> 1;
@@ -2635,39 +2645,57 @@ static bool fx_applies(const PassTuning* pm, unsigned nm) {
          !pm->overlap && !pm->slab_pipe && !pm->zf_pipe && !pm->fuse_stage;
 }
 
+static dim3 fx_zgrid(const Geom& g, const DevTables<double>& tb, int lgt, int pruned, unsigned nm) {
+  return pruned ? dim3(tb.nztl[lgt], nm) : dim3((g.nh + (1 << lgt) - 1) >> lgt, g.ny, nm);
+}
+// Fewer z tiles than two per SM (grids up to 128^3): the six lines of the inverse pass go on the grid and
+// the forward pass takes narrow tiles (us, z inverse and forward: 64^3 42 -> 14 and 32 -> 23, 128^3 67 -> 44
+// and 52 -> 34).
+static bool fx_few_tiles(const dim3& zgrid) { return (size_t)zgrid.x * zgrid.y * zgrid.z < (size_t)2 * device_sms(); }
+
+// Passes 1 and 2 into w (and the reset of the exponent maxima).
+static int fx_uw(const Geom& g, const DevTables<double>& tb, void* const a[3], void* const w[6], int pruned,
+                 const PassTuning* pm, cudaStream_t s, LaunchHook hook, void* hctx, unsigned nm, long long fxs,
+                 long long mstride) {
+  const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
+  int rc = (int)(nm > 1 ? cudaMemset2DAsync(ex.mz, (size_t)fxs * sizeof(int), kFxUnsetByte, ex.max_bytes, nm, s)
+                        : cudaMemsetAsync(ex.mz, kFxUnsetByte, ex.max_bytes, s));
+  if (rc) return rc;
+  const int lgt = fx_lg_tile(g.lnz), smem = strided_rows(g.nz) * (16 << lgt);
+  const dim3 zgrid = fx_zgrid(g, tb, lgt, pruned, nm);
+  Ptr6 pa{}, pw{};
+  for (int i = 0; i < 6; ++i) pw.p[i] = w[i];
+  for (int i = 0; i < 3; ++i) pa.p[i] = a[i];
+  const bool few = fx_few_tiles(zgrid);
+  const dim3 zigrid(zgrid.x, zgrid.y, few ? (pruned ? 6 : 6 * nm) : zgrid.z);
+  GT_HOOK(kKZinvCurl, true);
+#define GT_L(LG) \
+  k_fx_zinv<LG><<<zigrid, kFxTileThreads, smem, s>>>(pa, pw, tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
+  GT_DISPATCH_LG(g.lnz, GT_L)
+#undef GT_L
+  GT_HOOK(kKZinvCurl, false);
+  if ((rc = (int)cudaGetLastError())) return rc;
+  return fx_spass<0>(g, w, 6, tb.fwy, s, hook, hctx, ex, pruned ? tb.xa : g.nh, pruned ? 1 : 0, tb.xcut, (int)nm, fxs,
+                     mstride);
+}
+
 static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], void* const bcor[3],
                   void* const out[3], void* const w[6], int mode, int pruned, const PassTuning* pm, cudaStream_t s,
                   LaunchHook hook, void* hctx, const Batch<double>& bb) {
   const unsigned nm = bb.nmem > 0 ? (unsigned)bb.nmem : 1u;
   const long long mstride = bb.nmem > 0 ? bb.mstride : 0, fxs = nm > 1 ? pm->fx_stride : 0;
-  const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
-  int rc = (int)(nm > 1 ? cudaMemset2DAsync(ex.mz, (size_t)fxs * sizeof(int), kFxUnsetByte, ex.max_bytes, nm, s)
-                        : cudaMemsetAsync(ex.mz, kFxUnsetByte, ex.max_bytes, s));
+  int rc = fx_uw(g, tb, a, w, pruned, pm, s, hook, hctx, nm, fxs, mstride);
   if (rc) return rc;
+  const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
   const int lgt = fx_lg_tile(g.lnz), zsmem = strided_rows(g.nz) * (16 << lgt);
-  const dim3 zgrid = pruned ? dim3(tb.nztl[lgt], nm) : dim3((g.nh + (1 << lgt) - 1) >> lgt, g.ny, nm);
-  Ptr6 pa{}, pw{}, pb{}, po{};
+  const dim3 zgrid = fx_zgrid(g, tb, lgt, pruned, nm);
+  Ptr6 pw{}, pb{}, po{};
   for (int i = 0; i < 6; ++i) pw.p[i] = w[i];
   for (int i = 0; i < 3; ++i) {
-    pa.p[i] = a[i];
     pb.p[i] = bcor[i];
     po.p[i] = out[i];
   }
-  // fewer tiles than two per SM (grids up to 128^3): the six lines of the inverse pass on the grid,
-  // narrow tiles for the forward one (us, z inverse and forward: 64^3 42 -> 14 and 32 -> 23, 128^3 67 -> 44 and
-  // 52 -> 34)
-  const bool few = (size_t)zgrid.x * zgrid.y * zgrid.z < (size_t)2 * device_sms();
-  const dim3 zigrid(zgrid.x, zgrid.y, few ? (pruned ? 6 : 6 * nm) : zgrid.z);
-  GT_HOOK(kKZinvCurl, true);
-#define GT_L(LG) \
-  k_fx_zinv<LG><<<zigrid, kFxTileThreads, zsmem, s>>>(pa, pw, tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
-  GT_DISPATCH_LG(g.lnz, GT_L)
-#undef GT_L
-  GT_HOOK(kKZinvCurl, false);
-  if ((rc = (int)cudaGetLastError())) return rc;
   const int xlim = pruned ? tb.xa : g.nh;
-  if ((rc = fx_spass<0>(g, w, 6, tb.fwy, s, hook, hctx, ex, xlim, pruned ? 1 : 0, tb.xcut, (int)nm, fxs, mstride)))
-    return rc;
   {
     // whole warps: 96 threads (32 / (nx / 8) pairs) up to nx = 256, one pair above; ny nz / 2 is a multiple
     const long long npairs = (long long)g.ny * g.nz / 2;
@@ -2684,7 +2712,7 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
   if ((rc = fx_spass<1>(g, w, 3, tb.fwy, s, hook, hctx, ex, xlim, pruned ? 2 : 0, tb.xcut, (int)nm, fxs, mstride)))
     return rc;
   GT_HOOK(kKZFwdEpi, true);
-  if (few && g.lnz <= 7) {
+  if (fx_few_tiles(zgrid) && g.lnz <= 7) {
     const int lgn = lgt - 2;
     const dim3 ngrid = pruned ? dim3(tb.nztl[lgn], nm) : dim3((g.nh + (1 << lgn) - 1) >> lgn, g.ny, nm);
 #define GT_L(LG)                                                                                               \
@@ -3148,87 +3176,111 @@ int launch_pack_rows(const Geom& g, void* packed, void* field, int to_working, v
   return (int)cudaGetLastError();
 }
 
+// x transforms of nf fields between spectral rows (kx < xa read) and real rows.
 template <typename R>
-int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* spec, void* real_out,
-                   void* const w[6], void* stream, LaunchHook hook, void* hctx) {
+static int x_fields(const Geom& g, const DevTables<R>& tb, void* const* spec, void* const* real, int nf, int xa,
+                    bool inverse, const PassTuning* pm, cudaStream_t s, LaunchHook hook, void* hctx) {
+  const int csize = sizeof(Cplx<R>);
+  Ptr6 ps{}, pr{};
+  for (int i = 0; i < nf; ++i) {
+    ps.p[i] = spec[i];
+    pr.p[i] = real[i];
+  }
+  GT_HOOK(kKFft1, true);
+#ifdef GT_KERNELS_FX
+  const int P = xpass_pairs(g, 1, csize, 256, 1), threads = P * (g.nx / 8), smem = P * strided_rows(g.nx) * 16;
+  const dim3 grid((unsigned)((long long)g.ny * g.nz / 2 / P), nf);
+  const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
+#define GT_L(LG)                                                                                   \
+  if (inverse)                                                                                     \
+    k_fx_xc2r<LG><<<grid, threads, smem, s>>>(ps, pr, g, tb.fwx, P, xa, ex);                        \
+  else                                                                                             \
+    k_fx_xr2c<LG><<<grid, threads, smem, s>>>(pr, ps, g, tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
+#else
+  (void)pm;
+  const int P = xpass_pairs(g, 1, csize, max_threads<R>(), 1), threads = P * (g.nx / 8), smem = P * g.nx * csize;
+  const dim3 grid((unsigned)((long long)g.ny * g.nz / 2 / P), nf);
+  const R shalf = (R)(0.5 / ((double)g.nx * g.ny * g.nz));
+#define GT_L(LG)                                                                    \
+  if (inverse)                                                                      \
+    k_xc2r<R, LG><<<grid, threads, smem, s>>>(ps, pr, g, tb.twx, P, xa);             \
+  else                                                                              \
+    k_xr2c<R, LG><<<grid, threads, smem, s>>>(pr, ps, g, tb.twx, P, shalf);
+#endif
+  GT_DISPATCH_LG(g.lnx, GT_L)
+#undef GT_L
+  GT_HOOK(kKFft1, false);
+  return (int)cudaGetLastError();
+}
+
+// nf <= 6 fields at a time: one launch per axis.  pruned: the spectra are zero
+// outside the kept set, whose columns alone are transformed.  The spectra are
+// overwritten.
+template <typename R>
+int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* const* spec, void* const* real, int nf, int pruned,
+                   const PassTuning* pm, void* stream, LaunchHook hook, void* hctx) {
   int rc = set_smem_attrs<R>();
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  void* f[1] = {spec};
+  const int xlim = pruned ? tb.xa : g.nh;
 #ifdef GT_KERNELS_FX
-  // fixed point, the line exponents in w[2] (no caller keeps a field there)
-  const FxExp ex = fx_exp(w[2], g.ny, g.nz, g.nhp);
+  const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
   if ((rc = (int)cudaMemsetAsync(ex.mz, kFxUnsetByte, ex.max_bytes, s))) return rc;
-  if ((rc = fx_spass<2>(g, f, 1, tb.fwz, s, hook, hctx, ex))) return rc;
-  if ((rc = fx_spass<0>(g, f, 1, tb.fwy, s, hook, hctx, ex))) return rc;
-  const int P = xpass_pairs(g, 1, 16, 256, 1);
-  GT_HOOK(kKFft1, true);
-#define GT_L(LG)                                                                                  \
-k_fx_xc2r<LG><<<(unsigned)((long long)g.ny * g.nz / 2 / P), P * (g.nx / 8), P * strided_rows(g.nx) * 16, s>>>( \
-    spec, reinterpret_cast<double*>(real_out), g, tb.fwx, P, ex);
-  GT_DISPATCH_LG(g.lnx, GT_L)
-#undef GT_L
-  GT_HOOK(kKFft1, false);
-  return (int)cudaGetLastError();
+  if ((rc = fx_spass<2>(g, spec, nf, tb.fwz, s, hook, hctx, ex, xlim, pruned ? 3 : 0, tb.xcut))) return rc;
+  if ((rc = fx_spass<0>(g, spec, nf, tb.fwy, s, hook, hctx, ex, xlim, pruned ? 1 : 0, tb.xcut))) return rc;
 #else
-  (void)w;
-  if ((rc = spass<R>(g, f, 1, tb.twz, 2, +1, s, hook, hctx))) return rc;
-  if ((rc = spass<R>(g, f, 1, tb.twy, 1, +1, s, hook, hctx))) return rc;
-  const int csize = sizeof(Cplx<R>);
-  const int P = xpass_pairs(g, 1, csize, max_threads<R>(), 1);
-  const int LP = g.nx;
-  const long long nblocks = (long long)g.ny * g.nz / 2 / P;
-  GT_HOOK(kKFft1, true);
-#define GT_L(LG)                                                                    \
-  k_xc2r<R, LG><<<(unsigned)nblocks, P * (g.nx / 8), P * LP * csize, s>>>(            \
-      spec, reinterpret_cast<R*>(real_out), g, tb.twx, P);
-  GT_DISPATCH_LG(g.lnx, GT_L)
-#undef GT_L
-  GT_HOOK(kKFft1, false);
-  return (int)cudaGetLastError();
+  const bool pairs = sizeof(R) == 4;   // two columns per thread, tiles of 8 (as the pass of a step)
+  if ((rc = spass<R>(g, spec, nf, tb.twz, 2, +1, s, hook, hctx, xlim, pruned ? 3 : 0, tb.xcut, pairs ? 8 : 0, pairs)))
+    return rc;
+  if ((rc = spass<R>(g, spec, nf, tb.twy, 1, +1, s, hook, hctx, xlim, pruned ? 1 : 0, tb.xcut, pairs ? 8 : 0, pairs)))
+    return rc;
 #endif
+  return x_fields<R>(g, tb, spec, real, nf, xlim, true, pm, s, hook, hctx);
 }
 
 template <typename R>
-int launch_fft_dir(const Geom& g, const DevTables<R>& tb, const void* real_in, void* spec_out,
-                   void* const w[6], void* stream, LaunchHook hook, void* hctx) {
+int launch_fft_dir(const Geom& g, const DevTables<R>& tb, void* const* real, void* const* spec, int nf,
+                   const PassTuning* pm, void* stream, LaunchHook hook, void* hctx) {
   int rc = set_smem_attrs<R>();
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
 #ifdef GT_KERNELS_FX
-  const FxExp ex = fx_exp(w[2], g.ny, g.nz, g.nhp);   // as in launch_fft_inv
+  const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
   if ((rc = (int)cudaMemsetAsync(ex.mz, kFxUnsetByte, ex.max_bytes, s))) return rc;
-  const int P = xpass_pairs(g, 1, 16, 256, 1);
-  GT_HOOK(kKFft1, true);
-#define GT_L(LG)                                                                                  \
-k_fx_xr2c<LG><<<(unsigned)((long long)g.ny * g.nz / 2 / P), P * (g.nx / 8), P * strided_rows(g.nx) * 16, s>>>( \
-    reinterpret_cast<const double*>(real_in), spec_out, g, tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
-  GT_DISPATCH_LG(g.lnx, GT_L)
-#undef GT_L
-  GT_HOOK(kKFft1, false);
-  if ((rc = (int)cudaGetLastError())) return rc;
-  void* f[1] = {spec_out};
-  if ((rc = fx_spass<1>(g, f, 1, tb.fwy, s, hook, hctx, ex))) return rc;
-  return fx_spass<3>(g, f, 1, tb.fwz, s, hook, hctx, ex);
-#else
-  (void)w;
-  const int csize = sizeof(Cplx<R>);
-  const int P = xpass_pairs(g, 1, csize, max_threads<R>(), 1);
-  const int LP = g.nx;
-  const long long nblocks = (long long)g.ny * g.nz / 2 / P;
-  const R shalf = (R)(0.5 / ((double)g.nx * g.ny * g.nz));
-  GT_HOOK(kKFft1, true);
-#define GT_L(LG)                                                                    \
-  k_xr2c<R, LG><<<(unsigned)nblocks, P * (g.nx / 8), P * LP * csize, s>>>(            \
-      reinterpret_cast<const R*>(real_in), spec_out, g, tb.twx, P, shalf);
-  GT_DISPATCH_LG(g.lnx, GT_L)
-#undef GT_L
-  GT_HOOK(kKFft1, false);
-  if ((rc = (int)cudaGetLastError())) return rc;
-  void* f[1] = {spec_out};
-  if ((rc = spass<R>(g, f, 1, tb.twy, 1, -1, s, hook, hctx))) return rc;
-  return spass<R>(g, f, 1, tb.twz, 2, -1, s, hook, hctx);
 #endif
+  if ((rc = x_fields<R>(g, tb, spec, real, nf, g.nh, false, pm, s, hook, hctx))) return rc;
+#ifdef GT_KERNELS_FX
+  if ((rc = fx_spass<1>(g, spec, nf, tb.fwy, s, hook, hctx, ex))) return rc;
+  return fx_spass<3>(g, spec, nf, tb.fwz, s, hook, hctx, ex);
+#else
+  const bool pairs = sizeof(R) == 4;
+  if ((rc = spass<R>(g, spec, nf, tb.twy, 1, -1, s, hook, hctx, -1, 0, nullptr, pairs ? 8 : 0, pairs))) return rc;
+  return spass<R>(g, spec, nf, tb.twz, 2, -1, s, hook, hctx, -1, 0, nullptr, pairs ? 8 : 0, pairs);
+#endif
+}
+
+// u = curl a and w = k^2 a in physical space: passes 1 and 2 of a nonlinear
+// term (into w6) and the x transforms of its six fields.
+template <typename R>
+int launch_phys_uw(const Geom& g, const DevTables<R>& tb, void* const a[3], void* const w6[6], void* const u[3],
+                   void* const w[3], int pruned, const PassTuning* pm, int* err, void* stream, LaunchHook hook,
+                   void* hctx) {
+  int rc = set_smem_attrs<R>();
+  if (rc) return rc;
+  cudaStream_t s = (cudaStream_t)stream;
+  const int xlim = pruned ? tb.xa : g.nh;
+#ifdef GT_KERNELS_FX
+  (void)err;
+  if ((rc = fx_uw(g, tb, a, w6, pruned, pm, s, hook, hctx, 1, 0, 0))) return rc;
+#else
+  PassTuning def;   // the default form of the passes, whatever the step's knobs
+  if (pm) def.z_tma = pm->z_tma & 3;
+  if ((rc = nlt_phases<R>(g, tb, a, a, a, w6, kNltOnly, pruned, &def, err, stream, hook, hctx, 1))) return rc;
+  if ((rc = spass<R>(g, w6, 6, tb.twy, 1, +1, s, hook, hctx, xlim, pruned ? 1 : 0, tb.xcut, 8, sizeof(R) == 4)))
+    return rc;
+#endif
+  void* const out[6] = {u[0], u[1], u[2], w[0], w[1], w[2]};
+  return x_fields<R>(g, tb, w6, out, 6, xlim, true, pm, s, hook, hctx);
 }
 
 template <typename R>
@@ -3381,10 +3433,12 @@ const char* kernel_kind_name(int k) {
   template int launch_convert<R>(const Geom&, const void*, void*, int, void*, LaunchHook,      \
                                  void*);                                                        \
   template int launch_pack_rows<R>(const Geom&, void*, void*, int, void*, LaunchHook, void*);   \
-  template int launch_fft_inv<R>(const Geom&, const DevTables<R>&, void*, void*, void* const*, \
-                                 void*, LaunchHook, void*);                                     \
-  template int launch_fft_dir<R>(const Geom&, const DevTables<R>&, const void*, void*,         \
-                                 void* const*, void*, LaunchHook, void*);                       \
+  template int launch_fft_inv<R>(const Geom&, const DevTables<R>&, void* const*, void* const*, int, int, \
+                                 const PassTuning*, void*, LaunchHook, void*);                  \
+  template int launch_fft_dir<R>(const Geom&, const DevTables<R>&, void* const*, void* const*, int, \
+                                 const PassTuning*, void*, LaunchHook, void*);                  \
+  template int launch_phys_uw<R>(const Geom&, const DevTables<R>&, void* const*, void* const*, void* const*, \
+                                 void* const*, int, const PassTuning*, int*, void*, LaunchHook, void*); \
   template int launch_point<R>(const Geom&, const DevTables<R>&, void* const*, int, double*,   \
                                int, void*, LaunchHook, void*);                                  \
   template int launch_energy<R>(const Geom&, const DevTables<R>&, void* const*, int, double*, int, \
