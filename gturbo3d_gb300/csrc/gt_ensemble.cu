@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "gt_fft.cuh"
+#include "gt_fixed.cuh"
 #include "gt_handle.h"
 #include "gt_internal.h"
 
@@ -34,6 +35,7 @@ struct EnsClass {
   std::vector<int> members;     // ensemble indices; member k's fields are slab part k
   void* slab = nullptr;         // members x 12 fields
   void* btab = nullptr;         // members' emk tables, then their (omega, dt, dt2)
+  void* fx = nullptr;           // FP64: the members' line exponents, fx_stride ints apart
   int emk_len = 0;
   size_t scal_off = 0;          // byte offset of the scalars in btab
   cudaStream_t stream = nullptr;
@@ -88,6 +90,7 @@ void free_ensemble(gt_ensemble* e) {
     if (c.d_count) cudaFree(c.d_count);
     if (c.d_step) cudaFree(c.d_step);
     if (c.btab) cudaFree(c.btab);
+    if (c.fx) cudaFree(c.fx);
     if (c.slab) cudaFree(c.slab);
     if (c.join) cudaEventDestroy(c.join);
     if (c.stream) cudaStreamDestroy(c.stream);
@@ -311,6 +314,19 @@ int gt_ensemble_create(int32_t n, const gt_params* members, gt_ensemble** out) {
                                    static_cast<char*>(c.slab) + k * 12 * fbytes);
       if (rc) { free_ensemble(e); return rc; }
       if (e->m[c.members[k]]->g.field_elems() * esz != fbytes) { free_ensemble(e); return GT_EINVAL; }
+    }
+    if (p0.precision == GT_PREC_FP64) {
+      // batched fixed-point passes: the exponents of all members in one block, member 0's
+      // handle (whose knobs the class's launches use) pointing at it
+      gt_handle* h0 = e->m[c.members[0]];
+      const size_t stride = (fx_exp_ints(h0->g.ny, h0->g.nz, h0->g.nhp) + 63) / 64 * 64;
+      ce = cudaMalloc(&c.fx, c.members.size() * stride * sizeof(int));
+      if (ce != cudaSuccess) {
+        free_ensemble(e);
+        return ce == cudaErrorMemoryAllocation ? GT_ENOMEM : cuda_fail(ce, "line exponents");
+      }
+      h0->pm.fx_scratch = c.fx;
+      h0->pm.fx_stride = (long long)stride;
     }
   }
   for (int i = 0; i < n; ++i) {
