@@ -117,6 +117,23 @@ template <int SIGN, typename R> __device__ __forceinline__ CTrip<R> twmul(CTrip<
 }
 
 // ---- 64-bit fixed point (longlong2) ---------------------------------------
+// Opaque to the front end, which would re-associate a butterfly's integer sums.
+__device__ __forceinline__ i64 add64(i64 a, i64 b) {
+  i64 r;
+  asm("add.s64 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ i64 sub64(i64 a, i64 b) {
+  i64 r;
+  asm("sub.s64 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+template <> __device__ __forceinline__ longlong2 cadd<longlong2>(longlong2 a, longlong2 b) {
+  return longlong2{add64(a.x, b.x), add64(a.y, b.y)};
+}
+template <> __device__ __forceinline__ longlong2 csub<longlong2>(longlong2 a, longlong2 b) {
+  return longlong2{sub64(a.x, b.x), sub64(a.y, b.y)};
+}
 // a * b + c, 32 x 32 -> 64 bits: one instruction of the integer multiply pipe.
 __device__ __forceinline__ i64 mad_wide(int a, int b, i64 c) {
   i64 r;
@@ -148,8 +165,8 @@ template <int SIGN> __device__ __forceinline__ longlong2 twmul(longlong2 a, int4
   mi = mad_wide(i.x0, w.x, mi);
   const int r4 = r.x1 << (2 - f), i4 = i.x1 << (2 - f);
   longlong2 o;
-  o.x = mad_wide(i4, n1, mad_wide(r4, w.x, mr >> (30 + f)));
-  o.y = mad_wide(i4, w.x, mad_wide(r4, s1, mi >> (30 + f)));
+  o.x = mad_wide(i4, n1, mad_wide(r4, w.x, 0)) + (mr >> (30 + f));
+  o.y = mad_wide(i4, w.x, mad_wide(r4, s1, 0)) + (mi >> (30 + f));
   return o;
 }
 // sqrt(1/2) x, rounded, |x| < 2^62: the constant in Q63 as c1 2^32 + c0, the
@@ -181,22 +198,12 @@ template <int SIGN, typename C> __device__ __forceinline__ void dft4(C& x0, C& x
 // forward), and the radix-2 combination e +- o of such a product written
 // component-wise so that the products fuse into FMAs.
 template <int SIGN, typename R> __device__ __forceinline__ Cplx<R> w8_1(Cplx<R> o) {
-  if constexpr (std::is_same_v<R, i64>) {
-    return SIGN < 0 ? Cplx<R>{sqrt_half(o.x + o.y), sqrt_half(o.y - o.x)}
-                    : Cplx<R>{sqrt_half(o.x - o.y), sqrt_half(o.x + o.y)};
-  } else {
-    const R c = (R)0.70710678118654752440;
-    return SIGN < 0 ? Cplx<R>{c * (o.x + o.y), c * (o.y - o.x)} : Cplx<R>{c * (o.x - o.y), c * (o.x + o.y)};
-  }
+  const R c = (R)0.70710678118654752440;
+  return SIGN < 0 ? Cplx<R>{c * (o.x + o.y), c * (o.y - o.x)} : Cplx<R>{c * (o.x - o.y), c * (o.x + o.y)};
 }
 template <int SIGN, typename R> __device__ __forceinline__ Cplx<R> w8_3(Cplx<R> o) {
-  if constexpr (std::is_same_v<R, i64>) {
-    return SIGN < 0 ? Cplx<R>{sqrt_half(o.y - o.x), -sqrt_half(o.x + o.y)}
-                    : Cplx<R>{-sqrt_half(o.x + o.y), sqrt_half(o.x - o.y)};
-  } else {
-    const R c = (R)0.70710678118654752440;
-    return SIGN < 0 ? Cplx<R>{c * (o.y - o.x), -c * (o.x + o.y)} : Cplx<R>{-c * (o.x + o.y), c * (o.x - o.y)};
-  }
+  const R c = (R)0.70710678118654752440;
+  return SIGN < 0 ? Cplx<R>{c * (o.y - o.x), -c * (o.x + o.y)} : Cplx<R>{-c * (o.x + o.y), c * (o.x - o.y)};
 }
 template <typename C> __device__ __forceinline__ C fadd(C e, C o) { return C{e.x + o.x, e.y + o.y}; }
 template <typename C> __device__ __forceinline__ C fsub(C e, C o) { return C{e.x - o.x, e.y - o.y}; }
@@ -240,6 +247,43 @@ template <int SIGN, typename R, typename C> __device__ __forceinline__ void dft8
   v[1] = fadd(e1, o1); v[5] = fsub(e1, o1);
   v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
   v[3] = fadd(e3, o3); v[7] = fsub(e3, o3);
+}
+
+// The same butterflies in 64-bit fixed point, rotations folded into the signs
+// of the sums.
+template <int SIGN>
+__device__ __forceinline__ void fx_dft4(longlong2& x0, longlong2& x1, longlong2& x2, longlong2& x3) {
+  const longlong2 s0 = cadd(x0, x2), d0 = csub(x0, x2), s1 = cadd(x1, x3), t = csub(x1, x3);
+  x0 = cadd(s0, s1);
+  x2 = csub(s0, s1);
+  const longlong2 p{add64(d0.x, t.y), sub64(d0.y, t.x)}, q{sub64(d0.x, t.y), add64(d0.y, t.x)};   // d0 -+ i t
+  x1 = SIGN < 0 ? p : q;
+  x3 = SIGN < 0 ? q : p;
+}
+template <int SIGN> __device__ __forceinline__ void fx_dft8(longlong2 v[8]) {
+  longlong2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
+  longlong2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
+  fx_dft4<SIGN>(e0, e1, e2, e3);
+  fx_dft4<SIGN>(o0, o1, o2, o3);
+  v[0] = cadd(e0, o0);
+  v[4] = csub(e0, o0);
+  // W8 o1 = (sum1, dif1) or (dif1, sum1), W8^3 o3 = (dif3, -sum3) or (-sum3, dif3)
+  const i64 sum1 = sqrt_half(add64(o1.x, o1.y)), sum3 = sqrt_half(add64(o3.x, o3.y));
+  const i64 dif1 = sqrt_half(SIGN < 0 ? sub64(o1.y, o1.x) : sub64(o1.x, o1.y));
+  const i64 dif3 = sqrt_half(SIGN < 0 ? sub64(o3.y, o3.x) : sub64(o3.x, o3.y));
+  const longlong2 w1 = SIGN < 0 ? longlong2{sum1, dif1} : longlong2{dif1, sum1};
+  v[1] = cadd(e1, w1);
+  v[5] = csub(e1, w1);
+  const longlong2 p{add64(e2.x, o2.y), sub64(e2.y, o2.x)}, q{sub64(e2.x, o2.y), add64(e2.y, o2.x)};   // e2 -+ i o2
+  v[2] = SIGN < 0 ? p : q;
+  v[6] = SIGN < 0 ? q : p;
+  if (SIGN < 0) {
+    v[3] = longlong2{add64(e3.x, dif3), sub64(e3.y, sum3)};
+    v[7] = longlong2{sub64(e3.x, dif3), add64(e3.y, sum3)};
+  } else {
+    v[3] = longlong2{sub64(e3.x, sum3), add64(e3.y, dif3)};
+    v[7] = longlong2{add64(e3.x, sum3), sub64(e3.y, dif3)};
+  }
 }
 
 // Offset, within the per-stage twiddle table, of the stage that starts after

@@ -126,34 +126,46 @@ template <int O0, int O1, int NQ> struct FxRed {
 
 // ---- the line transform ---------------------------------------------------
 // Exchange scratch of TX interleaved lines (a strided tile's columns, or one x
-// line), one padding row after every 8: element e of the caller's line at
-// (e + e / 8) TX.  Every access of a stage is one base plus a compile-time
-// offset, and the 8 lanes of a 128-byte phase touch different banks.
+// line): the real parts' plane, then the imaginary parts', one padding row after
+// every 8: element e of the caller's line at (e + e / 8) TX of each plane.  Every
+// access of a stage is one base plus a compile-time offset.  Separate 8-byte
+// parts rather than 16-byte pairs: a pair's store wants four consecutive
+// registers, and the moves into them were 5 of 207 instructions a point.
 template <int LGL, int TX> struct FxMem {
-  longlong2* s;   // the scratch plus the line's column
+  i64* s;   // the scratch plus the line's column
   static constexpr int T = 1 << (LGL - 3);
   static constexpr int kRows = strided_rows(1 << LGL);
+  static constexpr int kPlane = kRows * TX;        // imaginary part of the element at s[o]: s[o + kPlane]
+  static constexpr int kWords = 2 * kPlane;
   // position j of the radix-8 butterfly of thread t in the stage after 2^LGNS points
-  template <int LGNS> __device__ __forceinline__ longlong2* bfly(int t) const {
-    if constexpr (LGNS == 0) {
-      return s + 9 * TX * t;
-    } else {
-      const int e = ((t >> LGNS) << (LGNS + 3)) + (t & ((1 << LGNS) - 1));
-      return s + TX * (e + (e >> 3));
+  template <int LGNS> __device__ __forceinline__ void put8(int t, const longlong2 v[8]) const {
+    constexpr int step = LGNS == 0 ? TX : TX * ((1 << LGNS) + (1 << LGNS) / 8);
+    const int e = ((t >> LGNS) << (LGNS + 3)) + (t & ((1 << LGNS) - 1));
+    i64* const p = s + (LGNS == 0 ? 9 * TX * t : TX * (e + (e >> 3)));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      p[j * step] = v[j].x;
+      p[j * step + kPlane] = v[j].y;
     }
   }
-  template <int LGNS> static constexpr int step() { return LGNS == 0 ? TX : TX * ((1 << LGNS) + (1 << LGNS) / 8); }
-  __device__ __forceinline__ longlong2& at(int e) const { return s[TX * (e + (e >> 3))]; }
-  // this thread's positions t + i T
+  static __device__ __forceinline__ int at(int e) { return TX * (e + (e >> 3)); }
+  // f(i, o) for this thread's positions t + i T, at s[o]
   template <typename F> __device__ __forceinline__ void own(int t, F&& f) const {
     if constexpr (T >= 8) {
-      longlong2* const p = s + TX * (t + (t >> 3));
+      const int o = at(t);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f(i, p[i * TX * (T + T / 8)]);
+      for (int i = 0; i < 8; ++i) f(i, o + i * TX * (T + T / 8));
     } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i) f(i, at(t + i * T));
     }
+  }
+  __device__ __forceinline__ longlong2 get(int o) const { return longlong2{s[o], s[o + kPlane]}; }
+  __device__ __forceinline__ void put_own(int t, const longlong2 v[8]) const {
+    own(t, [&](int i, int o) {
+      s[o] = v[i].x;
+      s[o + kPlane] = v[i].y;
+    });
   }
 };
 
@@ -183,13 +195,11 @@ __device__ __forceinline__ void fx_stages(longlong2 v[8], int t, const int4* __r
     one(v[0]);
 #pragma unroll
     for (int j = 1; j < 8; ++j) mul(v[j], &tws[(j - 1) * NS]);
-    dft8<SIGN, i64>(v);
+    fx_dft8<SIGN>(v);
     if constexpr (REM > LR) {
-      longlong2* const p = mem.template bfly<LGNS>(t);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) p[j * FxMem<LGL, TX>::template step<LGNS>()] = v[j];
+      mem.template put8<LGNS>(t, v);
       sync();
-      mem.own(t, [&](int i, const longlong2& q) { v[i] = q; });
+      mem.own(t, [&](int i, int o) { v[i] = mem.get(o); });
       sync();
       fx_stages<SIGN, LGL, LGNS + LR, TX>(v, t, tw, mem, sync, f);
     }
@@ -201,7 +211,7 @@ __device__ __forceinline__ void fx_stages(longlong2 v[8], int t, const int4* __r
       mul(v[m + 2], q);
       mul(v[m + 4], q + NS);
       mul(v[m + 6], q + 2 * NS);
-      dft4<SIGN>(v[m], v[m + 2], v[m + 4], v[m + 6]);
+      fx_dft4<SIGN>(v[m], v[m + 2], v[m + 4], v[m + 6]);
     }
   } else if constexpr (LR == 1) {
 #pragma unroll
@@ -228,7 +238,7 @@ __device__ __forceinline__ int fx_line(longlong2 v[8], int t, const int4* __rest
                                        const FxMem<LGL, TX>& mem, const Sync& sync, const Red& red) {
   if constexpr (LGL == 3) {
     // one stage, a thread's own line: the shift its outputs need (0 to 2)
-    dft8<SIGN, i64>(v);
+    fx_dft8<SIGN>(v);
     const int s = max(0, (64 - kFxOut) - __clz((int)fx_or_hi(v)));
     const i64 half = (1ll << s) >> 1;
 #pragma unroll
@@ -241,10 +251,8 @@ __device__ __forceinline__ int fx_line(longlong2 v[8], int t, const int4* __rest
     for (int i = 0; i < 8; ++i) acc += fx_abs_hi(v[i].x) + fx_abs_hi(v[i].y);
     acc = red.wsum((acc >> 7) + 1);
     if (red.lead) atomicAdd(red.sum(red.par), acc);
-    dft8<SIGN, i64>(v);
-    longlong2* const p = mem.template bfly<0>(t);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) p[j * TX] = v[j];
+    fx_dft8<SIGN>(v);
+    mem.template put8<0>(t, v);
     sync();
     // L1 < (total + 8) 2^39 -> below 2^61 with 2^33 to spare for roundings
     const int s = max(0, 10 - __clz((int)(*red.sum(red.par) + 8u)));
@@ -254,7 +262,8 @@ __device__ __forceinline__ int fx_line(longlong2 v[8], int t, const int4* __rest
     }
     const int s1 = max(min(s, fx_fold_need(LGL)), s - 2);
     const i64 half = (1ll << s1) >> 1;
-    mem.own(t, [&](int i, const longlong2& q) {
+    mem.own(t, [&](int i, int o) {
+      const longlong2 q = mem.get(o);
       v[i].x = shr_clamp(q.x + half, s1);
       v[i].y = shr_clamp(q.y + half, s1);
     });

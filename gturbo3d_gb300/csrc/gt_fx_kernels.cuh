@@ -65,7 +65,8 @@ k_fx_zinv(Ptr6 a, Ptr6 w, DevTables<double> tb, Geom g, int pruned, const int32_
   __syncthreads();
   const double kx = valid ? tb.fkx[X] : 0.0, kxs = valid ? tb.fkxs[X] : 0.0;
   const double ky = tb.fky[y], kys = tb.fkys[y];
-  const FxMem<LGZ, TX> mem_{reinterpret_cast<E*>(smraw) + x};
+  const FxMem<LGZ, TX> mem_{reinterpret_cast<i64*>(smraw) + x};
+  const size_t zstep = (size_t)T * plane;   // from a thread's position to its next
 #pragma unroll 1
   for (int f = f0; f < f1; ++f) {
     // the fields output f reads: u_0 <- (a1, a2), u_1 <- (a2, a0), u_2 <- (a0, a1); w_c <- a_c.
@@ -74,16 +75,18 @@ k_fx_zinv(Ptr6 a, Ptr6 w, DevTables<double> tb, Geom g, int pruned, const int32_
     const C* p2 = reinterpret_cast<const C*>(a.at(f == 0 ? 2 : f - 1));
     C d[8];
     unsigned h = 0;
+    p1 += base + (size_t)t * plane;
+    p2 += base + (size_t)t * plane;
+    const int32_t* cut = tb.xcut + (size_t)t * g.ny + y;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 8; ++i, p1 += zstep, p2 += zstep, cut += T * g.ny) {
       const int z = t + i * T;
-      const int lim = valid ? (pruned ? tb.xcut[(size_t)z * g.ny + y] : g.nh) : 0;
+      const int lim = valid ? (pruned ? *cut : g.nh) : 0;
       d[i] = C{0, 0};
       if (X < lim) {
-        const size_t o = (size_t)z * plane + base;
-        const C q = p1[o];
+        const C q = *p1;
         if (f < 3) {
-          const C r = p2[o];
+          const C r = *p2;
           const double kz = tb.fkz[z];
           const double k1 = f == 0 ? ky : (f == 1 ? kz : kx), k2 = f == 0 ? kz : (f == 1 ? kx : ky);
           d[i] = C{-k1 * r.y + k2 * q.y, k1 * r.x - k2 * q.x};   // produ.f90:44-63
@@ -110,11 +113,10 @@ k_fx_zinv(Ptr6 a, Ptr6 w, DevTables<double> tb, Geom g, int pruned, const int32_
     top = fx_top_get<LGZ>(red, top, 0);
     red.par ^= 1;
     const int u = fx_headroom(top);
-    E* out = reinterpret_cast<E*>(w.at(f));
+    E* out = reinterpret_cast<E*>(w.at(f)) + base + (size_t)t * plane;
     if (valid) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        out[(size_t)(t + i * T) * plane + base] = E{shl_clamp(v[i].x, u), shl_clamp(v[i].y, u)};
+      for (int i = 0; i < 8; ++i, out += zstep) *out = E{shl_clamp(v[i].x, u), shl_clamp(v[i].y, u)};
       if (t == 0) {
         if (e < kFxNaN / 2) e -= u;
         ex.ez[mem * fxs + ((size_t)f * g.ny + y) * g.nhp + X] = e;
@@ -154,6 +156,9 @@ k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim
   red.clear_all();
   const long long xo = mem * fxs;
   const int Xc = valid ? X : 0;
+  // element t of the line, and the step to t + T, t + 2 T, ...
+  E* const p0 = p + base + (size_t)t * (size_t)ls;
+  const size_t pstep = (size_t)T * (size_t)ls;
   E v[8];
   int e;
   if constexpr (KIND == 2) {
@@ -161,7 +166,7 @@ k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim
     unsigned h = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      d[i] = valid ? reinterpret_cast<const double2*>(p)[base + (size_t)(t + i * T) * (size_t)ls] : double2{0, 0};
+      d[i] = valid ? reinterpret_cast<const double2*>(p0)[i * pstep] : double2{0, 0};
       h = max(h, max(fx_abs_hi(d[i].x), fx_abs_hi(d[i].y)));
     }
     int em = (int)(h >> 20);
@@ -197,14 +202,13 @@ k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim
     e = top >= kFxNaN / 2 ? kFxNaN : top + (kFxOut - kFxIn);
     if constexpr (LGL > 3) __syncthreads();   // the slots are clear
   }
-  const FxMem<LGL, TX> mem_{reinterpret_cast<E*>(smraw) + x};
+  const FxMem<LGL, TX> mem_{reinterpret_cast<i64*>(smraw) + x};
   e += fx_line<SIGN>(v, t, reinterpret_cast<const int4*>(twv), mem_, BlockSync{}, red);
   if constexpr (KIND == 3) {
     if (valid) {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        reinterpret_cast<double2*>(p)[base + (size_t)(t + i * T) * (size_t)ls] =
-            double2{fx_to_double(v[i].x, e), fx_to_double(v[i].y, e)};
+        reinterpret_cast<double2*>(p0)[i * pstep] = double2{fx_to_double(v[i].x, e), fx_to_double(v[i].y, e)};
     }
   } else {
     unsigned mag = fx_top_put<LGL>(red, fx_or_hi(v), 0);
@@ -213,11 +217,8 @@ k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim
     const int u = fx_headroom(mag);
     if (valid) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = t + i * T;
-        if (ymask != 2 || X < xcut0[r])
-          p[base + (size_t)r * (size_t)ls] = E{shl_clamp(v[i].x, u), shl_clamp(v[i].y, u)};
-      }
+      for (int i = 0; i < 8; ++i)
+        if (ymask != 2 || X < xcut0[t + i * T]) p0[i * pstep] = E{shl_clamp(v[i].x, u), shl_clamp(v[i].y, u)};
       if (t == 0) {
         if (e < kFxNaN / 2) e -= u;
         if constexpr (KIND == 0) {
@@ -288,7 +289,7 @@ template <bool SWAP, int LGN>
 __device__ __forceinline__ void fx_split(const FxMem<LGN, 1>& mem, int t, int xa, int u, longlong2* oa, longlong2* ob) {
   constexpr int N = 1 << LGN, T = N / 8;
   for (int k = t; k < xa; k += T) {
-    longlong2 a = mem.at(k), b = mem.at((N - k) & (N - 1));
+    longlong2 a = mem.get(mem.at(k)), b = mem.get(mem.at((N - k) & (N - 1)));
     if (SWAP) {
       a = longlong2{a.y, a.x};
       b = longlong2{b.y, b.x};
@@ -317,16 +318,16 @@ k_fx_x(Ptr6 w, Geom g, const void* twv, int xa, int lgscale, FxExp ex, long long
   const size_t nhp = g.nhp;
   const size_t mo = member_offset(mstride, blockIdx.y);
   const long long xo = (long long)blockIdx.y * fxs;
-  E* const lines = reinterpret_cast<E*>(smraw) + p * 3 * LN;
-  const FxMem<LGN, 1> mem{lines + q * LN};
+  i64* const lines = reinterpret_cast<i64*>(smraw) + p * 6 * LN;   // three lines of two planes
+  const FxMem<LGN, 1> mem{lines + q * 2 * LN};
   auto red = fx_red_rows<LGN, NQ>(slots, gid, t);
   red.clear_all();
   __syncthreads();
   const int z = (int)((2 * pair) >> g.lny), y0 = (int)((2 * pair) & (size_t)(g.ny - 1));
   // component q of u x w (produ.f90:14-16), u = (z0.x, z0.y, z1.x), w = (z1.y, z2.x, z2.y):
-  // q = 0: uy wz - uz wy, 1: uz wx - ux wz, 2: ux wy - uy wx, as 64-bit words of the three lines
-  const int c_u1 = q == 0 ? 1 : (q == 1 ? 2 * LN : 0), c_w1 = q == 0 ? 4 * LN + 1 : (q == 1 ? 2 * LN + 1 : 4 * LN);
-  const int c_u2 = q == 0 ? 2 * LN : (q == 1 ? 0 : 1), c_w2 = q == 0 ? 4 * LN : (q == 1 ? 4 * LN + 1 : 2 * LN + 1);
+  // q = 0: uy wz - uz wy, 1: uz wx - ux wz, 2: ux wy - uy wx, as planes of the three lines
+  const int c_u1 = LN * (q == 0 ? 1 : (q == 1 ? 2 : 0)), c_w1 = LN * (q == 0 ? 5 : (q == 1 ? 3 : 4));
+  const int c_u2 = LN * (q == 0 ? 2 : (q == 1 ? 0 : 1)), c_w2 = LN * (q == 0 ? 4 : (q == 1 ? 5 : 3));
   E v[8];
   i64 c0[8];
   auto run = [&](auto sync) {
@@ -354,7 +355,7 @@ k_fx_x(Ptr6 w, Geom g, const void* twv, int xa, int lgscale, FxExp ex, long long
         hx |= fx_abs_hi(v[i].x);
         hy |= fx_abs_hi(v[i].y);
       }
-      mem.own(t, [&](int i, E& o) { o = v[i]; });
+      mem.put_own(t, v);
       if (r == 2) {
         const unsigned mag = fx_top_put<LGN>(red, hx | hy, 0);
         sync();
@@ -393,8 +394,8 @@ k_fx_x(Ptr6 w, Geom g, const void* twv, int xa, int lgscale, FxExp ex, long long
       red.par ^= 1;
       const FxMem<LGN, 1> all{lines};
       auto product = [&](auto shift) {
-        all.own(t, [&](int i, const E& l) {
-          const i64* b = &l.x;
+        all.own(t, [&](int i, int o) {
+          const i64* b = lines + o;
           const i64 c = fx_det(Limbs(shift(b[c_u1], s_u1)), Limbs(shift(b[c_w1], s_w1)), Limbs(shift(b[c_u2], s_u2)),
                                Limbs(shift(b[c_w2], s_w2)));
           if (r == 0) {
@@ -451,7 +452,7 @@ k_fx_xc2r(Ptr6 specs, Ptr6 reals, Geom g, const void* twv, int P, int xa, FxExp 
   for8([&](auto I) { v[I] = fx_pack_c2r<I, N>(X1, X2, e1, e1, top, t, xa); });
   int e = top >= kFxNaN / 2 ? kFxNaN : top + (kFxOut - kFxIn + 1);
   __syncthreads();
-  const FxMem<LGN, 1> mem{reinterpret_cast<E*>(smraw) + p * LN};
+  const FxMem<LGN, 1> mem{reinterpret_cast<i64*>(smraw) + p * 2 * LN};
   e += fx_line<+1>(v, t, reinterpret_cast<const int4*>(twv), mem, BlockSync{}, red);
   double* r0 = real + (2 * pair) * (size_t)N;
   double* r1 = r0 + N;
@@ -496,9 +497,9 @@ k_fx_xr2c(Ptr6 reals, Ptr6 specs, Geom g, const void* twv, int P, int lgscale, F
   E v[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = E{fx_from_double(d[i].x, em), fx_from_double(d[i].y, em)};
-  const FxMem<LGN, 1> mem{reinterpret_cast<E*>(smraw) + p * LN};
+  const FxMem<LGN, 1> mem{reinterpret_cast<i64*>(smraw) + p * 2 * LN};
   int e = fx_exponent(em) + fx_line<-1>(v, t, reinterpret_cast<const int4*>(twv), mem, BlockSync{}, red);
-  mem.own(t, [&](int i, E& o) { o = v[i]; });
+  mem.put_own(t, v);
   const unsigned mag = fx_top_put<LGN>(red, fx_or_hi(v), 0);
   __syncthreads();
   const int u = fx_headroom(fx_top_get<LGN>(red, mag, 0));
@@ -523,7 +524,7 @@ k_fx_xr2c(Ptr6 reals, Ptr6 specs, Geom g, const void* twv, int P, int lgscale, F
 // (e' e as one factor would save six more, but its rounding repeats every step:
 // 100 steps at 64^3 were off by 4.3e-15 instead of 0.9e-15.)
 template <int LGT, int TX>
-__device__ __forceinline__ void fx_epilogue(longlong2* __restrict__ sm, int reg, const int e[3], int t, int X, int y,
+__device__ __forceinline__ void fx_epilogue(i64* __restrict__ sm, int reg, const int e[3], int t, int X, int y,
                                             int ylim, size_t base, size_t plane, const Ptr6& bc, const Ptr6& out,
                                             const DevTables<double>& tb, const Geom& g, int mode, int pruned) {
   using C = double2;
@@ -542,7 +543,7 @@ __device__ __forceinline__ void fx_epilogue(longlong2* __restrict__ sm, int reg,
     if (X >= (pruned ? zlim : ylim)) continue;        // written columns: the kept ones, or all of the row's
     const size_t o = (size_t)z * plane + base;
     const C b0 = b0p[o], b1 = b1p[o], b2 = b2p[o];
-    const longlong2* const n = &mem.at(z);
+    const int n = mem.at(z);
     const double kz = tb.fkz[z], okz = tb.omega * kz;
     const bool zero_mode = (X == 0) && (y == 0) && (z == 0);
     double em = 1.0, ik2;
@@ -555,7 +556,7 @@ __device__ __forceinline__ void fx_epilogue(longlong2* __restrict__ sm, int reg,
       if (mode != kNltOnly) em = tb.emk[((size_t)z * g.ny + y) * g.nh + X];
     }
     auto val = [&](int f, const C& b) {   // v + i omega kz b(t)
-      const longlong2 q = n[f * reg];
+      const longlong2 q = mem.get(n + f * reg);
       return C{fx_to_double(q.x, e[f]) - okz * b.y, fx_to_double(q.y, e[f]) + okz * b.x};
     };
     C a0 = val(0, b0), a1 = val(1, b1), a2 = val(2, b2);
@@ -610,7 +611,7 @@ k_fx_zfwd(Ptr6 w, Ptr6 bc, Ptr6 out, DevTables<double> tb, Geom g, int mode, int
   const unsigned mem = pruned ? blockIdx.y : blockIdx.z;
   member_tables(bt, mem, tb);
   const size_t base = (size_t)y * g.nhp + (valid ? X : 0) + member_offset(bt.mstride, mem);
-  constexpr int reg = strided_rows(1 << LGZ) * TX;
+  constexpr int reg = FxMem<LGZ, TX>::kWords;
   const int4* tw = reinterpret_cast<const int4*>(tb.fwz);
   const long long xo = (long long)mem * fxs;
   auto red = fx_red_tile<TX>(slots, x, t);
@@ -620,27 +621,27 @@ k_fx_zfwd(Ptr6 w, Ptr6 bc, Ptr6 out, DevTables<double> tb, Geom g, int mode, int
   int e[3];
 #pragma unroll 1
   for (int f = 0; f < 3; ++f) {
-    E* S = reinterpret_cast<E*>(smraw) + f * reg;
-    const E* in = reinterpret_cast<const E*>(w.at(f));
+    i64* S = reinterpret_cast<i64*>(smraw) + f * reg;
+    const E* in = reinterpret_cast<const E*>(w.at(f)) + base + (size_t)t * plane;
+    const int* er = ex.eyf + xo + ((size_t)f * g.nz + t) * g.nhp + (valid ? X : 0);
     const int top = ex.myf[xo + (size_t)f * g.nhp + (valid ? X : 0)];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int z = t + i * T;
-      const int sh = top - (valid ? ex.eyf[xo + ((size_t)f * g.nz + z) * g.nhp + X] : 0) + (kFxOut - kFxIn);
-      const E q = valid ? in[(size_t)z * plane + base] : E{0, 0};
+    for (int i = 0; i < 8; ++i, in += (size_t)T * plane, er += T * g.nhp) {
+      const int sh = top - (valid ? *er : 0) + (kFxOut - kFxIn);
+      const E q = valid ? *in : E{0, 0};
       v[i] = E{shr_clamp(q.x, sh), shr_clamp(q.y, sh)};
     }
     const FxMem<LGZ, TX> mem_{S + x};
     int ef = top >= kFxNaN / 2 ? kFxNaN : top + (kFxOut - kFxIn);
     ef += fx_line<-1>(v, t, tw, mem_, BlockSync{}, red);
     red.par ^= 1;
-    mem_.own(t, [&](int i, E& o) { o = v[i]; });
+    mem_.put_own(t, v);
     if (f == 0) e[0] = ef;
     if (f == 1) e[1] = ef;
     if (f == 2) e[2] = ef;
   }
   if (!valid) return;   // no barrier follows
-  fx_epilogue<LGZ, TX>(reinterpret_cast<E*>(smraw) + x, reg, e, t, X, y, ylim, base, plane, bc, out, tb, g, mode,
+  fx_epilogue<LGZ, TX>(reinterpret_cast<i64*>(smraw) + x, reg, e, t, X, y, ylim, base, plane, bc, out, tb, g, mode,
                        pruned);
 }
 
