@@ -38,6 +38,7 @@ template <int LGZ>
 __global__ void __launch_bounds__(kFxTileThreads, 3)
 k_fx_zinv(Ptr6 a, Ptr6 w, DevTables<double> tb, Geom g, int pruned, const int32_t* __restrict__ tiles,
           int split, FxExp ex, long long fxs, long long mstride) {
+  pass_enter();
   using C = double2;
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -135,6 +136,7 @@ template <int KIND, int LGL>
 __global__ void __launch_bounds__(kFxTileThreads, 3)
 k_fx_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int xlim, int ymask,
            const int32_t* __restrict__ xcut0, int nf, FxExp ex, long long fxs, long long mstride) {
+  pass_enter();
   using E = longlong2;
   constexpr int SIGN = (KIND == 0 || KIND == 2) ? +1 : -1;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -304,6 +306,7 @@ template <int LGN> constexpr int fx_x_threads() { return LGN <= 8 ? 96 : 3 << (L
 template <int LGN>
 __global__ void __launch_bounds__(fx_x_threads<LGN>(), 768 / fx_x_threads<LGN>())
 k_fx_x(Ptr6 w, Geom g, const void* twv, int xa, int lgscale, FxExp ex, long long fxs, long long mstride) {
+  pass_enter();
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int N = 1 << LGN, T = N / 8, NQ = 2, LN = FxMem<LGN, 1>::kRows;
@@ -433,6 +436,7 @@ k_fx_x(Ptr6 w, Geom g, const void* twv, int xa, int lgscale, FxExp ex, long long
 template <int LGN>
 __global__ void __launch_bounds__(256)
 k_fx_xc2r(Ptr6 specs, Ptr6 reals, Geom g, const void* twv, int P, int xa, FxExp ex) {
+  pass_enter();
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ unsigned slots[FxRowRed<LGN, 1>::kSlots];
@@ -466,6 +470,7 @@ k_fx_xc2r(Ptr6 specs, Ptr6 reals, Geom g, const void* twv, int P, int xa, FxExp 
 template <int LGN>
 __global__ void __launch_bounds__(256)
 k_fx_xr2c(Ptr6 reals, Ptr6 specs, Geom g, const void* twv, int P, int lgscale, FxExp ex) {
+  pass_enter();
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ unsigned slots[FxRowRed<LGN, 1>::kSlots];
@@ -594,6 +599,7 @@ template <int LGZ, int TX>
 __global__ void __launch_bounds__(TX << (LGZ - 3), 512 / (TX << (LGZ - 3)))
 k_fx_zfwd(Ptr6 w, Ptr6 bc, Ptr6 out, DevTables<double> tb, Geom g, int mode, int pruned,
           const int32_t* __restrict__ tiles, FxExp ex, long long fxs, Batch<double> bt) {
+  pass_enter();
   using E = longlong2;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ unsigned slots[FxTileRed<TX>::kSlots];

@@ -150,10 +150,11 @@ __device__ __forceinline__ void load_cols_async(ColT<R, W>* sdst, const Cplx<R>*
 template <typename R> constexpr int zcols() { return sizeof(R) == 4 ? 2 : 1; }
 template <typename R> constexpr int zfwd_cols() { return 1; }
 
-template <typename R, int LGZ>
+template <typename R, int LGZ, bool DEP = false>
 __global__ void __launch_bounds__(max_threads<R>() / zcols<R>())
 k_zinv_curl(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, const int32_t* __restrict__ tiles,
             int k2part, long long mstride) {
+  if (DEP) pass_enter();
   using C = Cplx<R>;
   constexpr int W = zcols<R>();
   using E = ColT<R, W>;
@@ -688,10 +689,11 @@ k_zk2(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, const int32
 // pass's time (mixed, us: 64^3, 43 tiles, 15.6 -> 13.0; 128 x 128 x 32, 85 tiles,
 // 15.4 -> 12.4; but 128^3, 221 tiles, 18.9 -> 21.2).
 // ---------------------------------------------------------------------------
-template <typename R, int LGZ>
+template <typename R, int LGZ, bool DEP = false>
 __global__ void __launch_bounds__(kSpassThreads, sizeof(R) == 8 ? 2 : 3)
 k_zinv_curl1(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, const int32_t* __restrict__ tiles,
              int split, long long mstride) {
+  if (DEP) pass_enter();
   using C = Cplx<R>;
   constexpr int W = zcols<R>();
   using E = ColT<R, W>;
@@ -827,10 +829,11 @@ k_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTX, i
 // The inverse y pass (six fields, loads masked by the truncation) runs best
 // at 4 resident blocks (64 registers, small spills), the forward one at 3
 // (80 registers): 0.90 / 0.36 ms at 512^3.
-template <int SIGN, int LGL>
+template <int SIGN, int LGL, bool DEP = false>
 __global__ void __launch_bounds__(kSpassThreads, SIGN > 0 ? 4 : 3)
 k_spass2(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTP, int xlim, int ymask,
          const int32_t* __restrict__ xcut0, int nf, long long mstride) {
+  if (DEP) pass_enter();
   using C = float2;
   using E = CPair<float>;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1217,9 +1220,10 @@ template <typename R> constexpr int xbatch_threads() { return sizeof(R) == 8 ? 1
 
 // PARK: row 0's products wait in a shared region (N complex + N real per
 // group) instead of registers, for 3 resident blocks instead of 2.
-template <typename R, int LGN, bool PARK = false>
+template <typename R, int LGN, bool PARK = false, bool DEP = false>
 __global__ void __launch_bounds__(xbatch_threads<R>(), PARK ? 3 : 2)
 k_xbatch(Ptr6 w, Geom g, const void* twv, R shalf, int xa, long long mstride) {
+  if (DEP) pass_enter();
   using C = Cplx<R>;
   using E = CTrip<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1398,10 +1402,11 @@ __device__ __forceinline__ void zfwd_epilogue(const ColT<R, W>* __restrict__ sm,
 // ---------------------------------------------------------------------------
 // Pass 5: forward z transform of three fields, then the spectral epilogue.
 // ---------------------------------------------------------------------------
-template <typename R, int LGZ>
+template <typename R, int LGZ, bool DEP = false>
 __global__ void __launch_bounds__(max_threads<R>() / zfwd_cols<R>())
 k_zfwd_epi(Ptr6 w, Ptr6 bc, Ptr6 out, DevTables<R> tb, Geom g, int lgTX, int mode, int pruned,
            const int32_t* __restrict__ tiles, Batch<R> bt) {
+  if (DEP) pass_enter();
   using C = Cplx<R>;
   constexpr int W = zfwd_cols<R>();
   using E = ColT<R, W>;
@@ -2036,6 +2041,7 @@ constexpr int kForceThreads = 128;
 template <typename R>
 __global__ void __launch_bounds__(kForceThreads)
 k_force_head(Ptr6 b, ForceHead* head, Geom g) {
+  pass_enter();
   using C = Cplx<R>;
   const int n = head->n, step = head->step;
   const ForceEntry* e = reinterpret_cast<const ForceEntry*>(head + 1) + (size_t)step * n;
@@ -2417,18 +2423,24 @@ static int set_smem_attrs() {
   int optin = 0;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return (int)e;
-  cudaError_t es[8 * 32 + 1];
+  cudaError_t es[8 * 40 + 1];
   int n = 0;
 #define GT_ALLOW(LG)                                     \
   es[n++] = allow_smem(k_zinv_curl<R, LG>, optin);       \
   es[n++] = allow_smem(k_zinv_curl_pf<R, LG>, optin);    \
   es[n++] = allow_smem(k_zk2<R, LG>, optin);             \
   es[n++] = allow_smem(k_zinv_curl1<R, LG>, optin);      \
+  es[n++] = allow_smem(k_zinv_curl<R, LG, sizeof(R) == 4>, optin);     \
+  es[n++] = allow_smem(k_zinv_curl1<R, LG, sizeof(R) == 4>, optin);    \
+  es[n++] = allow_smem(k_xbatch<R, LG, false, sizeof(R) == 4>, optin); \
+  es[n++] = allow_smem(k_zfwd_epi<R, LG, sizeof(R) == 4>, optin);      \
   es[n++] = allow_smem(k_spass<R, 1, LG>, optin);        \
   es[n++] = allow_smem(k_spass<R, -1, LG>, optin);       \
   if (sizeof(R) == 4) {                                  \
     es[n++] = allow_smem(k_spass2<1, LG>, optin);        \
     es[n++] = allow_smem(k_spass2<-1, LG>, optin);       \
+    es[n++] = allow_smem(k_spass2<1, LG, true>, optin);  \
+    es[n++] = allow_smem(k_spass2<-1, LG, true>, optin); \
     es[n++] = allow_smem(k_spass2_pf<1, LG>, optin);     \
     es[n++] = allow_smem(k_spass2_pf<-1, LG>, optin);    \
     es[n++] = allow_smem(k_zfwd_cl<(LG >= 4 ? LG : 4)>, optin); \
@@ -2519,6 +2531,36 @@ static int device_sms() {
   return nsm;
 }
 
+// Launches `dependent`, a form of the pass that begins with pass_enter, set up
+// while the stream's previous kernel ends (programmatic serialization), where
+// `apart` holds and the grid has up to kDependentBlocks blocks: 0.2-0.4 us less
+// per launch (ms per step without -> with: mixed 128x128x32 0.0760 -> 0.0725,
+// FP64 64^3 0.125 -> 0.123).  Beyond, that is lost in the kernel's time.  An
+// ensemble's batches take `plain`: in a graph of concurrent classes kernels that
+// hold the wait ran 3 % slower even without the attribute (12x64^3 + 4x128^3,
+// 64 steps: 47.4 -> 49.1 ms).
+constexpr size_t kDependentBlocks = 4096;
+
+template <typename... KA, typename... A>
+static void launch_pass(bool apart, void (*plain)(KA...), void (*dependent)(KA...), dim3 grid, unsigned threads,
+                        size_t smem, cudaStream_t s, A&&... args) {
+  if (!apart || (size_t)grid.x * grid.y * grid.z > kDependentBlocks) {
+    plain<<<grid, threads, smem, s>>>(static_cast<KA>(args)...);
+    return;
+  }
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, dependent, static_cast<KA>(args)...);   // errors through cudaGetLastError
+}
+
 // Launches F(LG) for the run-time log2 length lg (3..10).
 #define GT_DISPATCH_LG(lg, F)                                                  \
   switch (lg) {                                                                \
@@ -2588,10 +2630,10 @@ static int spass(const Geom& g, void* const* fields, int nf, const void* tw, int
       GT_HOOK(kind, true);
 #define GT_L(LG)                                                                                      \
   if (sign > 0)                                                                                       \
-    k_spass2<1, LG><<<grid2, c2.threads / 2, c2.smem, s>>>(f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, \
+    launch_pass(nmem == 1, k_spass2<1, LG>, k_spass2<1, LG, true>, grid2, c2.threads / 2, c2.smem, s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, \
                                                             nf, mstride);                                  \
   else                                                                                                \
-    k_spass2<-1, LG><<<grid2, c2.threads / 2, c2.smem, s>>>(f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, \
+    launch_pass(nmem == 1, k_spass2<-1, LG>, k_spass2<-1, LG, true>, grid2, c2.threads / 2, c2.smem, s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, \
                                                              nf, mstride);
       GT_DISPATCH_LG(lgL, GT_L)
 #undef GT_L
@@ -2630,7 +2672,7 @@ static int fx_spass(const Geom& g, void* const* fields, int nf, const void* tw, 
   const int kind = KIND == 0 || KIND == 2 ? kKYPass : kKYFwd;
   GT_HOOK(kind, true);
 #define GT_L(LG)                                                                                              \
-  k_fx_spass<KIND, LG><<<grid, kFxTileThreads, smem, s>>>(f, g, tw, ls, os, xlim, ymask, xcut0, nf, ex, fxs, mstride);
+  launch_pass(nmem == 1, k_fx_spass<KIND, LG>, k_fx_spass<KIND, LG>, grid, kFxTileThreads, smem, s, f, g, tw, ls, os, xlim, ymask, xcut0, nf, ex, fxs, mstride);
   GT_DISPATCH_LG(lgL, GT_L)
 #undef GT_L
   GT_HOOK(kind, false);
@@ -2670,7 +2712,7 @@ static int fx_uw(const Geom& g, const DevTables<double>& tb, void* const a[3], v
   const dim3 zigrid(zgrid.x, zgrid.y, few ? (pruned ? 6 : 6 * nm) : zgrid.z);
   GT_HOOK(kKZinvCurl, true);
 #define GT_L(LG) \
-  k_fx_zinv<LG><<<zigrid, kFxTileThreads, smem, s>>>(pa, pw, tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
+  launch_pass(nm == 1, k_fx_zinv<LG>, k_fx_zinv<LG>, zigrid, kFxTileThreads, smem, s, pa, pw, tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
   GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   GT_HOOK(kKZinvCurl, false);
@@ -2702,7 +2744,7 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
     const int P = g.nx >= 256 ? 1 : 256 / g.nx;
     GT_HOOK(kKXCross, true);
 #define GT_L(LG)                                                                                        \
-  k_fx_x<LG><<<dim3((unsigned)(npairs / P), nm), fx_x_threads<LG>(), 3 * P * strided_rows(g.nx) * 16, s>>>(              \
+  launch_pass(nm == 1, k_fx_x<LG>, k_fx_x<LG>, dim3((unsigned)(npairs / P), nm), fx_x_threads<LG>(), 3 * P * strided_rows(g.nx) * 16, s,               \
       pw, g, tb.fwx, xlim, g.lnx + g.lny + g.lnz, ex, fxs, mstride);
     GT_DISPATCH_LG(g.lnx, GT_L)
 #undef GT_L
@@ -2716,13 +2758,14 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
     const int lgn = lgt - 2;
     const dim3 ngrid = pruned ? dim3(tb.nztl[lgn], nm) : dim3((g.nh + (1 << lgn) - 1) >> lgn, g.ny, nm);
 #define GT_L(LG)                                                                                               \
-  k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4><<<ngrid, kFxTileThreads / 4, 3 * zsmem / 4, s>>>( \
+  launch_pass(nm == 1, k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>,                       \
+              k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>, ngrid, kFxTileThreads / 4, 3 * zsmem / 4, s,  \
       pw, pb, po, tb, g, mode, pruned, tb.ztl[lgn], ex, fxs, bb);
     GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   } else {
 #define GT_L(LG)                                                                                                \
-  k_fx_zfwd<LG, fx_tile<LG>()><<<zgrid, kFxTileThreads, 3 * zsmem, s>>>(pw, pb, po, tb, g, mode, pruned, tb.ztl[lgt], \
+  launch_pass(nm == 1, k_fx_zfwd<LG, fx_tile<LG>()>, k_fx_zfwd<LG, fx_tile<LG>()>, zgrid, kFxTileThreads, 3 * zsmem, s, pw, pb, po, tb, g, mode, pruned, tb.ztl[lgt], \
                                                                         ex, fxs, bb);
     GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
@@ -2829,13 +2872,15 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
       const int fs = few && !(pm && pm->z_split == 2);
       const dim3 gridf(grid.x, grid.y, fs ? (pruned ? 6 : 6 * nm) : grid.z);
 #define GT_L(LG)                                                                                    \
-  k_zinv_curl1<R, LG><<<gridf, c.threads / zcols<R>(), c.smem / 3, s>>>(pa, pw, tb, g, c.lgTX, pruned, \
+  launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl1<R, LG>, k_zinv_curl1<R, LG, sizeof(R) == 4>, gridf, c.threads / zcols<R>(), c.smem / 3, s, \
+              pa, pw, tb, g, c.lgTX, pruned, \
                                                                         tb.ztl[c.lgTX], fs, mstride);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
     } else {
 #define GT_L(LG)                                                                                   \
-  k_zinv_curl<R, LG><<<grid, c.threads / zcols<R>(), c.smem, s>>>(pa, pw, tb, g, c.lgTX, pruned,    \
+  launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl<R, LG>, k_zinv_curl<R, LG, sizeof(R) == 4>, grid, c.threads / zcols<R>(), c.smem, s, \
+              pa, pw, tb, g, c.lgTX, pruned,    \
                                                                   tb.ztl[c.lgTX], split ? 0 : 1, mstride);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
@@ -2897,7 +2942,8 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
       GT_HOOK(kKXCross, true);
       if (!pm || pm->x_fused == 2) {
 #define GT_L(LG) \
-  k_xbatch<R, LG><<<dim3((unsigned)(npairs / P), nm), P * T, 3 * smem, ms>>>(pw, gs, tb.twx, shalf, xlim, mstride);
+  launch_pass(sizeof(R) == 4 && nm == 1, k_xbatch<R, LG>, k_xbatch<R, LG, false, sizeof(R) == 4>, dim3((unsigned)(npairs / P), nm), P * T, 3 * smem, ms, \
+              pw, gs, tb.twx, shalf, xlim, mstride);
         GT_DISPATCH_LG(gs.lnx, GT_L)
 #undef GT_L
       } else if (pm->x_fused == 3) {
@@ -3033,7 +3079,8 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
 #undef GT_L
     } else {
 #define GT_L(LG)                                                                                   \
-  k_zfwd_epi<R, LG><<<grid, c.threads / zfwd_cols<R>(), c.smem, s>>>(pw, pb, po, tb, g, c.lgTX, mode, \
+  launch_pass(sizeof(R) == 4 && nm == 1, k_zfwd_epi<R, LG>, k_zfwd_epi<R, LG, sizeof(R) == 4>, grid, c.threads / zfwd_cols<R>(), c.smem, s, \
+              pw, pb, po, tb, g, c.lgTX, mode, \
                                                                  pruned, tb.ztl[c.lgTX], bb);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
@@ -3125,7 +3172,7 @@ int launch_force_head(const Geom& g, void* const b[3], ForceHead* head, void* st
   Ptr6 pb{};
   for (int i = 0; i < 3; ++i) pb.p[i] = b[i];
   GT_HOOK(kKForce, true);
-  k_force_head<R><<<1, kForceThreads, 0, (cudaStream_t)stream>>>(pb, head, g);
+  launch_pass(true, k_force_head<R>, k_force_head<R>, 1, kForceThreads, 0, (cudaStream_t)stream, pb, head, g);
   GT_HOOK(kKForce, false);
   return (int)cudaGetLastError();
 }
@@ -3193,9 +3240,9 @@ static int x_fields(const Geom& g, const DevTables<R>& tb, void* const* spec, vo
   const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
 #define GT_L(LG)                                                                                   \
   if (inverse)                                                                                     \
-    k_fx_xc2r<LG><<<grid, threads, smem, s>>>(ps, pr, g, tb.fwx, P, xa, ex);                        \
+    launch_pass(true, k_fx_xc2r<LG>, k_fx_xc2r<LG>, grid, threads, smem, s, ps, pr, g, tb.fwx, P, xa, ex);                        \
   else                                                                                             \
-    k_fx_xr2c<LG><<<grid, threads, smem, s>>>(pr, ps, g, tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
+    launch_pass(true, k_fx_xr2c<LG>, k_fx_xr2c<LG>, grid, threads, smem, s, pr, ps, g, tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
 #else
   (void)pm;
   const int P = xpass_pairs(g, 1, csize, max_threads<R>(), 1), threads = P * (g.nx / 8), smem = P * g.nx * csize;
