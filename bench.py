@@ -594,7 +594,7 @@ def run_ours(args):
             "fp64": {"value": fp64_value, "unit": UNIT, "steps": args.fp64_steps, "warmup": 3,
                      "e2e": {"value": fp64_e2e, "unit": UNIT, "steps": args.fp64_e2e_steps,
                              "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-                     "bound": "fp64 alu (DADD/DFMA issue; HBM is not the limit)", "alu_probe_ginst_s": alu},
+                     "bound": "instruction issue of the 64-bit fixed-point transforms (HBM is not the limit)", "alu_probe_ginst_s": alu},
             "rel_energy_err_mixed_vs_fp64": rel_err, "energy_steps": args.energy_steps,
             "roofline": roof, "clocks": clk}
     sim.close()

@@ -22,21 +22,11 @@
 
 namespace gt {
 
-// A transform's values are float2, or longlong2 in block fixed point (the
-// FP64 form, gt_fixed.cuh); double2 is the FP64 form's storage.
 using i64 = long long;
 template <typename R> struct CplxOf;
 template <> struct CplxOf<float> { using type = float2; };
 template <> struct CplxOf<double> { using type = double2; };
-template <> struct CplxOf<i64> { using type = longlong2; };
 template <typename R> using Cplx = typename CplxOf<R>::type;
-
-// A table twiddle e^{-2 pi i m / L}: a complex value, or for fixed-point
-// transforms cos and sin in Q62 as balanced 32-bit limbs {c1, c0, s1, s0}
-// (value c1 2^32 + c0, both signed).
-template <typename R> struct TwOf { using type = Cplx<R>; };
-template <> struct TwOf<i64> { using type = int4; };
-template <typename R> using Tw = typename TwOf<R>::type;
 
 template <typename C> __device__ __forceinline__ C cadd(C a, C b) { return C{a.x + b.x, a.y + b.y}; }
 template <typename C> __device__ __forceinline__ C csub(C a, C b) { return C{a.x - b.x, a.y - b.y}; }
@@ -117,6 +107,9 @@ template <int SIGN, typename R> __device__ __forceinline__ CTrip<R> twmul(CTrip<
 }
 
 // ---- 64-bit fixed point (longlong2) ---------------------------------------
+// Values are longlong2 in block fixed point; a table twiddle e^{-2 pi i m / L}
+// is cos and sin in Q62 as balanced 32-bit limbs {c1, c0, s1, s0} (value
+// c1 2^32 + c0, both signed).
 // Opaque to the front end, which would re-associate a butterfly's integer sums.
 __device__ __forceinline__ i64 add64(i64 a, i64 b) {
   i64 r;
@@ -315,10 +308,10 @@ template <typename R, int LGL, int LGNS> struct StageTw {
   static constexpr int NS = 1 << LGNS;
   static constexpr int T = 1 << (LGL - 3);
   static constexpr int N = LGNS == 0 ? 1 : (LR == 3 ? 7 : (LR == 2 ? 6 : 4));
-  Tw<R> w[N];
-  __device__ __forceinline__ void load(int t, const Tw<R>* __restrict__ tw) {
+  Cplx<R> w[N];
+  __device__ __forceinline__ void load(int t, const Cplx<R>* __restrict__ tw) {
     if constexpr (LGNS > 0) {
-      const Tw<R>* tws = tw + (1 << LGL) + tw_stage_offset(LGL, LGNS);
+      const Cplx<R>* tws = tw + (1 << LGL) + tw_stage_offset(LGL, LGNS);
       if constexpr (LR == 3) {
         const int k = t & (NS - 1);
 #pragma unroll
@@ -368,7 +361,7 @@ template <typename R, typename Idx> struct TripMem {
 // PF: twiddles a stage ahead (FP32 default: measured faster); otherwise at
 // the stage itself (FP64: the extra live registers spill in the z pass).
 template <int SIGN, typename R, int LGL, int LGNS, bool PF, typename E, typename Mem, typename Sync>
-__device__ __forceinline__ void fft_stages_ct(E v[8], int t, const Tw<R>* __restrict__ tw, const Mem& mem,
+__device__ __forceinline__ void fft_stages_ct(E v[8], int t, const Cplx<R>* __restrict__ tw, const Mem& mem,
                                               const Sync& sync, const StageTw<R, LGL, LGNS>& cur) {
   constexpr int REM = LGL - LGNS;
   constexpr int LR = REM >= 3 ? 3 : REM;

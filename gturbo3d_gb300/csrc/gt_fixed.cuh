@@ -3,10 +3,11 @@
 // GB300 issues 1.8 FP64 adds per clock and SM but 32 64-bit integer adds and
 // 25-32 32x32+64-bit multiply-adds, so a line is transformed as 64-bit
 // integers with one power-of-two scale per line instead of as doubles.  At
-// 256^3 (ms a launch, FP64 arithmetic -> this): z inverse 0.93 -> 0.27, y inverse
-// 1.54 -> 0.30, x 3.82 -> 0.84, y forward 0.77 -> 0.146, z forward 0.55 -> 0.214;
-// the RK2 step 15.2 -> 3.5 ms, and 132.4 -> 25.6 ms at 512^3.  The passes are bound by instruction issue (2.3-2.5 of 4 a clock) with the multiply pipe at
-// 57-64 % and the ALU pipe at 53-61 %; DRAM is at 13-29 %.
+// 256^3 (ms a launch, FP64 arithmetic -> this): z inverse 0.93 -> 0.25, y inverse
+// 1.54 -> 0.29, x 3.82 -> 0.83, y forward 0.77 -> 0.147, z forward 0.55 -> 0.197;
+// the RK2 step 15.2 -> 3.40 ms, and 132.4 -> 25.0 ms at 512^3.  The passes are
+// bound by instruction issue (2.2-2.5 of 4 a clock) with the multiply pipe at
+// 51-64 % and the ALU pipe at 50-62 %; DRAM is at 13-29 %.
 //
 // * A line's inputs are scaled so that every component is below 2^59
 //   (kFxIn bits); the first radix-8 stage adds at most 3.5 bits.

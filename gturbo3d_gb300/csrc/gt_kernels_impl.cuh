@@ -8,7 +8,7 @@
 //                     formed on load (produ.f90:44-63, nlt.f90:26-40), then
 //                     the inverse z transform of all six fields.
 //   2. k_spass2     : inverse y transform of the six fields, in place (FP32,
-//                     two columns per thread; k_spass for FP64).
+//                     two columns per thread; k_spass for FP64 arithmetic).
 //   3. k_xbatch     : per pair of (y,z) rows, the six C2R x transforms (two
 //                     fields per complex FFT, a row's three packed lines as
 //                     one three-line transform), u x w in registers
@@ -28,6 +28,9 @@
 // nonzero (tile lists for the z passes, kx < xa for the y and x passes).
 // Spectral fields are [nz][ny][nhp] complex, x fastest, rows padded to a
 // multiple of 128 bytes; columns nh..nhp-1 are never read or written.
+//
+// The FP64 form runs the same five passes on the integer pipe by default
+// (gt_fx_kernels.cuh, chosen by fx_applies): 132 -> 25 ms a step at 512^3.
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <atomic>
@@ -711,7 +714,8 @@ k_zinv_curl1(Ptr6 a, Ptr6 w, DevTables<R> tb, Geom g, int lgTX, int pruned, cons
   const bool valid = X0 < ylim;
   constexpr int T = 1 << (LGZ - 3);
   const size_t plane = (size_t)g.ny * g.nhp;
-  const size_t base = (size_t)y * g.nhp + (valid ? X0 : 0) + member_offset(mstride, pruned ? blockIdx.y : (split ? blockIdx.z / 6 : blockIdx.z));
+  const size_t base = (size_t)y * g.nhp + (valid ? X0 : 0) +
+                      member_offset(mstride, pruned ? blockIdx.y : (split ? blockIdx.z / 6 : blockIdx.z));
   const int f0 = split ? (int)(blockIdx.z % 6) : 0, f1 = split ? f0 + 1 : 6;
   const StridedIdxLg idx{lgTP, xp};
   const C* tw = reinterpret_cast<const C*>(tb.twz);
@@ -2453,9 +2457,7 @@ static int set_smem_attrs() {
   es[n++] = allow_smem(k_xbatch<R, LG, true>, optin);    \
   es[n++] = allow_smem(k_zfwd_epi<R, LG>, optin);        \
   es[n++] = allow_smem(k_zfwd_epi_pf<R, LG>, optin);     \
-  es[n++] = allow_smem(k_zfwd_zinv<R, LG>, optin);       \
-  es[n++] = allow_smem(k_xc2r<R, LG>, optin);            \
-  es[n++] = allow_smem(k_xr2c<R, LG>, optin);
+  es[n++] = allow_smem(k_zfwd_zinv<R, LG>, optin);
   GT_ALLOW(3) GT_ALLOW(4) GT_ALLOW(5) GT_ALLOW(6) GT_ALLOW(7) GT_ALLOW(8) GT_ALLOW(9) GT_ALLOW(10)
 #undef GT_ALLOW
 #ifdef GT_KERNELS_FX
@@ -2467,9 +2469,13 @@ static int set_smem_attrs() {
   es[n++] = allow_smem(k_fx_spass<3, LG>, optin); \
   es[n++] = allow_smem(k_fx_x<LG>, optin);        \
   es[n++] = allow_smem(k_fx_zfwd<LG, fx_tile<LG>()>, optin);
+#else
+#define GT_ALLOW(LG)                          \
+  es[n++] = allow_smem(k_xc2r<R, LG>, optin); \
+  es[n++] = allow_smem(k_xr2c<R, LG>, optin);
+#endif
   GT_ALLOW(3) GT_ALLOW(4) GT_ALLOW(5) GT_ALLOW(6) GT_ALLOW(7) GT_ALLOW(8) GT_ALLOW(9) GT_ALLOW(10)
 #undef GT_ALLOW
-#endif
   es[n++] = allow_smem(k_diag<R>, optin);
   for (int i = 0; i < n; ++i)
     if (es[i] != cudaSuccess) return (int)es[i];
@@ -2630,11 +2636,11 @@ static int spass(const Geom& g, void* const* fields, int nf, const void* tw, int
       GT_HOOK(kind, true);
 #define GT_L(LG)                                                                                      \
   if (sign > 0)                                                                                       \
-    launch_pass(nmem == 1, k_spass2<1, LG>, k_spass2<1, LG, true>, grid2, c2.threads / 2, c2.smem, s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, \
-                                                            nf, mstride);                                  \
+    launch_pass(nmem == 1, k_spass2<1, LG>, k_spass2<1, LG, true>, grid2, c2.threads / 2, c2.smem, \
+                s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, nf, mstride);                    \
   else                                                                                                \
-    launch_pass(nmem == 1, k_spass2<-1, LG>, k_spass2<-1, LG, true>, grid2, c2.threads / 2, c2.smem, s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, \
-                                                             nf, mstride);
+    launch_pass(nmem == 1, k_spass2<-1, LG>, k_spass2<-1, LG, true>, grid2, c2.threads / 2, c2.smem, \
+                s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, nf, mstride);
       GT_DISPATCH_LG(lgL, GT_L)
 #undef GT_L
       GT_HOOK(kind, false);
@@ -2672,7 +2678,8 @@ static int fx_spass(const Geom& g, void* const* fields, int nf, const void* tw, 
   const int kind = KIND == 0 || KIND == 2 ? kKYPass : kKYFwd;
   GT_HOOK(kind, true);
 #define GT_L(LG)                                                                                              \
-  launch_pass(nmem == 1, k_fx_spass<KIND, LG>, k_fx_spass<KIND, LG>, grid, kFxTileThreads, smem, s, f, g, tw, ls, os, xlim, ymask, xcut0, nf, ex, fxs, mstride);
+  launch_pass(nmem == 1, k_fx_spass<KIND, LG>, k_fx_spass<KIND, LG>, grid, kFxTileThreads, smem, \
+              s, f, g, tw, ls, os, xlim, ymask, xcut0, nf, ex, fxs, mstride);
   GT_DISPATCH_LG(lgL, GT_L)
 #undef GT_L
   GT_HOOK(kind, false);
@@ -2712,7 +2719,8 @@ static int fx_uw(const Geom& g, const DevTables<double>& tb, void* const a[3], v
   const dim3 zigrid(zgrid.x, zgrid.y, few ? (pruned ? 6 : 6 * nm) : zgrid.z);
   GT_HOOK(kKZinvCurl, true);
 #define GT_L(LG) \
-  launch_pass(nm == 1, k_fx_zinv<LG>, k_fx_zinv<LG>, zigrid, kFxTileThreads, smem, s, pa, pw, tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
+  launch_pass(nm == 1, k_fx_zinv<LG>, k_fx_zinv<LG>, zigrid, kFxTileThreads, smem, s, pa, pw, \
+              tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
   GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   GT_HOOK(kKZinvCurl, false);
@@ -2744,7 +2752,8 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
     const int P = g.nx >= 256 ? 1 : 256 / g.nx;
     GT_HOOK(kKXCross, true);
 #define GT_L(LG)                                                                                        \
-  launch_pass(nm == 1, k_fx_x<LG>, k_fx_x<LG>, dim3((unsigned)(npairs / P), nm), fx_x_threads<LG>(), 3 * P * strided_rows(g.nx) * 16, s,               \
+  launch_pass(nm == 1, k_fx_x<LG>, k_fx_x<LG>, dim3((unsigned)(npairs / P), nm), fx_x_threads<LG>(), \
+              3 * P * strided_rows(g.nx) * 16, s, \
       pw, g, tb.fwx, xlim, g.lnx + g.lny + g.lnz, ex, fxs, mstride);
     GT_DISPATCH_LG(g.lnx, GT_L)
 #undef GT_L
@@ -2759,14 +2768,14 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
     const dim3 ngrid = pruned ? dim3(tb.nztl[lgn], nm) : dim3((g.nh + (1 << lgn) - 1) >> lgn, g.ny, nm);
 #define GT_L(LG)                                                                                               \
   launch_pass(nm == 1, k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>,                       \
-              k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>, ngrid, kFxTileThreads / 4, 3 * zsmem / 4, s,  \
+              k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>, ngrid, kFxTileThreads / 4, 3 * zsmem / 4, s, \
       pw, pb, po, tb, g, mode, pruned, tb.ztl[lgn], ex, fxs, bb);
     GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   } else {
 #define GT_L(LG)                                                                                                \
-  launch_pass(nm == 1, k_fx_zfwd<LG, fx_tile<LG>()>, k_fx_zfwd<LG, fx_tile<LG>()>, zgrid, kFxTileThreads, 3 * zsmem, s, pw, pb, po, tb, g, mode, pruned, tb.ztl[lgt], \
-                                                                        ex, fxs, bb);
+  launch_pass(nm == 1, k_fx_zfwd<LG, fx_tile<LG>()>, k_fx_zfwd<LG, fx_tile<LG>()>, zgrid, kFxTileThreads,      \
+              3 * zsmem, s, pw, pb, po, tb, g, mode, pruned, tb.ztl[lgt], ex, fxs, bb);
     GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   }
@@ -2872,14 +2881,16 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
       const int fs = few && !(pm && pm->z_split == 2);
       const dim3 gridf(grid.x, grid.y, fs ? (pruned ? 6 : 6 * nm) : grid.z);
 #define GT_L(LG)                                                                                    \
-  launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl1<R, LG>, k_zinv_curl1<R, LG, sizeof(R) == 4>, gridf, c.threads / zcols<R>(), c.smem / 3, s, \
+  launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl1<R, LG>, k_zinv_curl1<R, LG, sizeof(R) == 4>, gridf, \
+              c.threads / zcols<R>(), c.smem / 3, s, \
               pa, pw, tb, g, c.lgTX, pruned, \
                                                                         tb.ztl[c.lgTX], fs, mstride);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
     } else {
 #define GT_L(LG)                                                                                   \
-  launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl<R, LG>, k_zinv_curl<R, LG, sizeof(R) == 4>, grid, c.threads / zcols<R>(), c.smem, s, \
+  launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl<R, LG>, k_zinv_curl<R, LG, sizeof(R) == 4>, grid, \
+              c.threads / zcols<R>(), c.smem, s, \
               pa, pw, tb, g, c.lgTX, pruned,    \
                                                                   tb.ztl[c.lgTX], split ? 0 : 1, mstride);
       GT_DISPATCH_LG(g.lnz, GT_L)
@@ -2942,7 +2953,8 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
       GT_HOOK(kKXCross, true);
       if (!pm || pm->x_fused == 2) {
 #define GT_L(LG) \
-  launch_pass(sizeof(R) == 4 && nm == 1, k_xbatch<R, LG>, k_xbatch<R, LG, false, sizeof(R) == 4>, dim3((unsigned)(npairs / P), nm), P * T, 3 * smem, ms, \
+  launch_pass(sizeof(R) == 4 && nm == 1, k_xbatch<R, LG>, k_xbatch<R, LG, false, sizeof(R) == 4>, \
+              dim3((unsigned)(npairs / P), nm), P * T, 3 * smem, ms, \
               pw, gs, tb.twx, shalf, xlim, mstride);
         GT_DISPATCH_LG(gs.lnx, GT_L)
 #undef GT_L
@@ -3079,7 +3091,8 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
 #undef GT_L
     } else {
 #define GT_L(LG)                                                                                   \
-  launch_pass(sizeof(R) == 4 && nm == 1, k_zfwd_epi<R, LG>, k_zfwd_epi<R, LG, sizeof(R) == 4>, grid, c.threads / zfwd_cols<R>(), c.smem, s, \
+  launch_pass(sizeof(R) == 4 && nm == 1, k_zfwd_epi<R, LG>, k_zfwd_epi<R, LG, sizeof(R) == 4>, grid, \
+              c.threads / zfwd_cols<R>(), c.smem, s, \
               pw, pb, po, tb, g, c.lgTX, mode, \
                                                                  pruned, tb.ztl[c.lgTX], bb);
       GT_DISPATCH_LG(g.lnz, GT_L)
@@ -3240,9 +3253,11 @@ static int x_fields(const Geom& g, const DevTables<R>& tb, void* const* spec, vo
   const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
 #define GT_L(LG)                                                                                   \
   if (inverse)                                                                                     \
-    launch_pass(true, k_fx_xc2r<LG>, k_fx_xc2r<LG>, grid, threads, smem, s, ps, pr, g, tb.fwx, P, xa, ex);                        \
+    launch_pass(true, k_fx_xc2r<LG>, k_fx_xc2r<LG>, grid, threads, smem, s, ps, pr, g, \
+                tb.fwx, P, xa, ex);                                                      \
   else                                                                                             \
-    launch_pass(true, k_fx_xr2c<LG>, k_fx_xr2c<LG>, grid, threads, smem, s, pr, ps, g, tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
+    launch_pass(true, k_fx_xr2c<LG>, k_fx_xr2c<LG>, grid, threads, smem, s, pr, ps, g, \
+                tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
 #else
   (void)pm;
   const int P = xpass_pairs(g, 1, csize, max_threads<R>(), 1), threads = P * (g.nx / 8), smem = P * g.nx * csize;
@@ -3477,8 +3492,6 @@ const char* kernel_kind_name(int k) {
   template int launch_force_batch<R>(const Geom&, void* const*, const Batch<R>&,                \
                                      const ForceEntry*, const int*, int, int, const int*, void*, \
                                      LaunchHook, void*);                                        \
-  template int launch_convert<R>(const Geom&, const void*, void*, int, void*, LaunchHook,      \
-                                 void*);                                                        \
   template int launch_pack_rows<R>(const Geom&, void*, void*, int, void*, LaunchHook, void*);   \
   template int launch_fft_inv<R>(const Geom&, const DevTables<R>&, void* const*, void* const*, int, int, \
                                  const PassTuning*, void*, LaunchHook, void*);                  \
@@ -3495,5 +3508,8 @@ const char* kernel_kind_name(int k) {
                               LaunchHook, void*);
 
 GT_INST(GT_REAL)
+#ifndef GT_KERNELS_FX   // only the mixed form has a working precision to convert to
+template int launch_convert<float>(const Geom&, const void*, void*, int, void*, LaunchHook, void*);
+#endif
 
 }  // namespace gt

@@ -1,8 +1,9 @@
 // ALU issue-rate probe: the FP64 and FP32 ceilings of the transform passes.
 //
-// The plain (FP64) form of the step is bound by the FP64 pipe, not by HBM, so
-// its roofline needs this GPU's FP64 add and fused multiply-add rates; they
-// are measured here rather than taken from a datasheet.  Each thread runs
+// Passes in FP64 arithmetic are bound by the FP64 pipe, not by HBM (the plain
+// form therefore transforms lines on the integer pipe), so their roofline needs
+// this GPU's FP64 add and fused multiply-add rates; they are measured here
+// rather than taken from a datasheet.  Each thread runs
 // eight independent dependency chains (enough to cover the pipe latency) over
 // a grid of 8 blocks of 256 threads per SM; rates are warp-instruction counts
 // times 32 lanes per second.

@@ -45,7 +45,11 @@ extern "C" {
 #define GT_DT2_AS_BUILT 0    /* dt2 = 0: rkstep.f90 reads a dt2 nothing assigns */
 #define GT_DT2_RK2 1         /* dt2 = dt/2: the RK2 midpoint the scheme intends  */
 
-#define GT_PREC_FP64 0       /* plain form: everything in FP64                    */
+#define GT_PREC_FP64 0       /* plain form: FP64 fields and pointwise work; line
+                              * transforms in 64-bit block fixed point, whose
+                              * error is below FP64 arithmetic's.  An input with
+                              * an infinity or NaN gives NaN in every value its
+                              * transforms reach; inputs below 2.3e-308 count as 0 */
 #define GT_PREC_MIXED 1      /* FP32 state, FFTs and products; FP64 exponentials,
                                 forcing normalisation and reductions             */
 
@@ -199,7 +203,7 @@ int gt_check_finite(gt_handle* h);
 int gt_set_pruning(gt_handle* h, int32_t enable);
 /* *active = 1 if the next gt_rk2_step takes the pruned path. */
 int gt_pruning_active(gt_handle* h, int32_t* active);
-/* Launch-shape tuning (results are unchanged):
+/* Launch-shape tuning (results are unchanged to rounding):
  * "y_tx", "z_tx" (0 = default, or 2/4/8/16: x-columns per block of the y / z passes;
  * the z default is 16 for FP32 z columns of 256 points or more, else 8),
  * "x_fused" (x pass: 2 = one thread group per row pair, the three packed lines
@@ -231,7 +235,10 @@ int gt_pruning_active(gt_handle* h, int32_t* active);
  * copies of the three fields with an mbarrier each; 1 the z forward pass, 2
  * the z inverse pass; both the default for z columns of 256 and 512 points;
  * 4, with 2, the z inverse pass's six outputs written by tensor stores, the
- * default for z columns of 256 points). */
+ * default for z columns of 256 points).  The plain form's default passes (fixed
+ * point) have tiles of their own: "y_tx" and "z_tx" have no effect on them, and a
+ * value of "x_fused", "z_split", "overlap", "slab_pipe", "zf_pipe" or "fuse_stage"
+ * other than the default runs the step in FP64 arithmetic. */
 int gt_set_tuning(gt_handle* h, const char* key, int32_t value);
 /* The current value of one gt_set_tuning knob (the per-grid default until
  * it is set). */
@@ -329,8 +336,8 @@ int gt_selftest_wait_timeout(gt_handle* h);
 
 /* Measures this GPU's ALU issue rates in G thread-instructions per second:
  * rates[0] DFMA, [1] DADD, [2] FFMA, [3] FADD (independent chains, 8 blocks of
- * 256 threads per SM).  The FP64 form of the step is FP64-ALU bound; these are
- * its roofline denominators.  No reference counterpart. */
+ * 256 threads per SM): the bound of passes in FP64 arithmetic, and the reason why
+ * the plain form transforms lines on the integer pipe.  No reference counterpart. */
 int gt_probe_alu(int32_t device, double* rates);
 
 /* Measures the DRAM rate that each pass's access pattern allows: copy kernels
