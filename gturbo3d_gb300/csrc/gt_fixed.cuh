@@ -5,9 +5,10 @@
 // integers with one power-of-two scale per line instead of as doubles.  At
 // 256^3 (ms a launch, FP64 arithmetic -> this): z inverse 0.93 -> 0.25, y inverse
 // 1.54 -> 0.29, x 3.82 -> 0.83, y forward 0.77 -> 0.147, z forward 0.55 -> 0.197;
-// the RK2 step 15.2 -> 3.40 ms, and 132.4 -> 25.0 ms at 512^3.  The passes are
-// bound by instruction issue (2.2-2.5 of 4 a clock) with the multiply pipe at
-// 51-64 % and the ALU pipe at 50-62 %; DRAM is at 13-29 %.
+// the RK2 step 15.2 -> 3.40 ms, and 132.4 -> 25.0 ms at 512^3.  The x and y
+// passes are bound by instruction issue (2.0-2.4 of 4 a clock) with the multiply
+// pipe at 46-59 % and the ALU pipe at 50-57 %, DRAM at 12-35 %; the z passes also
+// by their FP64 pointwise work (28-48 %) and spectral loads.
 //
 // * A line's inputs are scaled so that every component is below 2^59
 //   (kFxIn bits); the first radix-8 stage adds at most 3.5 bits.
