@@ -57,8 +57,9 @@ float rann(int32_t& irand);
 void draw_forcing(const gt_params& p, const HostTables& t, int32_t& seed,
                   std::vector<ForceEntry>& out);
 bool entries_unique(const ForceEntry* e, size_t n);
-// Faults in n host arrays of `bytes` each before device results are copied there.
-void prefault(double* const* dst, int n, size_t bytes);
+// Faults in n host arrays of `bytes` each before device results are copied there;
+// the bytes that were not there yet.
+size_t prefault(double* const* dst, int n, size_t bytes);
 
 // Resident forcing of a graph-replayed step: n entries a step follow the head;
 // the scatter kernel adds those of step `step` and advances it.
