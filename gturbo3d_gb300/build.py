@@ -39,8 +39,8 @@ def _newest_header() -> float:
 
 
 def _compile(src: Path, nvcc: str, hdr_time: float, verbose: bool) -> tuple[Path, str]:
-    obj = BUILD / (src.name + ".o")
-    if obj.exists() and obj.stat().st_mtime >= max(src.stat().st_mtime, hdr_time):
+    obj, log = BUILD / (src.name + ".o"), BUILD / (src.name + ".log")
+    if obj.exists() and log.exists() and obj.stat().st_mtime >= max(src.stat().st_mtime, hdr_time):
         return obj, ""
     if src.suffix == ".cu":
         cmd = [nvcc, *NVCC_FLAGS, "-c", str(src), "-o", str(obj)]
@@ -52,6 +52,7 @@ def _compile(src: Path, nvcc: str, hdr_time: float, verbose: bool) -> tuple[Path
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"compile failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+    log.write_text(r.stdout + r.stderr)   # registers and spills of every kernel, for the resource tests
     return obj, (r.stdout + r.stderr) if verbose else ""
 
 

@@ -1,0 +1,35 @@
+"""Registers and spills of the built kernels (the assembler's resource report, kept by the
+build beside each object) against what their launches count on."""
+import re
+
+import pytest
+
+REGISTERS = 65536   # per SM
+
+
+def resources(unit):
+    """{mangled kernel name: (registers, spill store bytes, spill load bytes)} of one unit."""
+    from gturbo3d_gb300 import build
+    build.build()
+    out, name, spills = {}, None, (0, 0)
+    for line in (build.BUILD / f"{unit}.log").read_text().splitlines():
+        if m := re.search(r"Compiling entry function '(\S+)'", line):
+            name = m.group(1)
+        elif m := re.search(r"(\d+) bytes spill stores, (\d+) bytes spill loads", line):
+            spills = (int(m.group(1)), int(m.group(2)))
+        elif (m := re.search(r"Used (\d+) registers", line)) and name:
+            out[name] = (int(m.group(1)), *spills)
+    return out
+
+
+def kernels(unit, prefix):
+    found = {k: v for k, v in resources(unit).items() if k.startswith(prefix)}
+    assert found
+    return found
+
+
+@pytest.mark.parametrize("unit", ["gt_kernels_f32.cu", "gt_kernels_f64.cu"])
+def test_diagnostics_run_two_blocks_per_sm(unit):
+    """The launch puts two blocks of 256 threads on every SM in one wave."""
+    for name, (regs, _, _) in kernels(unit, "_ZN2gt6k_diagI").items():
+        assert (regs + 7) // 8 * 8 * 256 * 2 <= REGISTERS, (name, regs)
