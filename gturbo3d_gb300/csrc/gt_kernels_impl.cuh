@@ -793,10 +793,6 @@ k_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTX, i
   const int TX = 1 << lgTX;
   const int x = threadIdx.x & (TX - 1), t = threadIdx.x >> lgTX;
   const int X = blockIdx.x * TX + x;
-  if (ymask == 3) {   // z pass over kept columns: X < xcut0[y]
-    xlim = min(xlim, xcut0[blockIdx.y]);
-    if ((int)blockIdx.x * TX >= xlim) return;
-  }
   const bool valid = X < xlim;
   constexpr int T = 1 << (LGL - 3);
   // blockIdx.z = member * nf + field
@@ -833,7 +829,10 @@ k_spass(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTX, i
 // The inverse y pass (six fields, loads masked by the truncation) runs best
 // at 4 resident blocks (64 registers, small spills), the forward one at 3
 // (80 registers): 0.90 / 0.36 ms at 512^3.
-template <int SIGN, int LGL, bool DEP = false>
+// KEPT: a z pass over the kept columns X < xcut0[y], a form of its own: as a run-time
+// case it cost the inverse y passes registers (128-point lines 32 -> 68 bytes of spill
+// stores; a step's inverse y pass at 256 x 128 x 256 with y_prefetch = 0, 0.058 -> 0.064 ms).
+template <int SIGN, int LGL, bool DEP = false, bool KEPT = false>
 __global__ void __launch_bounds__(kSpassThreads, SIGN > 0 ? 4 : 3)
 k_spass2(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTP, int xlim, int ymask,
          const int32_t* __restrict__ xcut0, int nf, long long mstride) {
@@ -845,7 +844,7 @@ k_spass2(Ptr6 f, Geom g, const void* twv, long long ls, long long os, int lgTP, 
   const int TP = 1 << lgTP;
   const int xp = threadIdx.x & (TP - 1), t = threadIdx.x >> lgTP;
   const int X0 = 2 * (blockIdx.x * TP + xp);
-  if (ymask == 3) {   // z pass over kept columns: X < xcut0[y]
+  if constexpr (KEPT) {
     xlim = min(xlim, xcut0[blockIdx.y]);
     if (2 * (int)blockIdx.x * TP >= xlim) return;
   }
@@ -2447,6 +2446,7 @@ static int set_smem_attrs() {
     es[n++] = allow_smem(k_spass2<1, LG>, optin);        \
     es[n++] = allow_smem(k_spass2<-1, LG>, optin);       \
     es[n++] = allow_smem(k_spass2<1, LG, true>, optin);  \
+    es[n++] = allow_smem(k_spass2<1, LG, true, true>, optin); \
     es[n++] = allow_smem(k_spass2<-1, LG, true>, optin); \
     es[n++] = allow_smem(k_spass2_pf<1, LG>, optin);     \
     es[n++] = allow_smem(k_spass2_pf<-1, LG>, optin);    \
@@ -2587,11 +2587,13 @@ static void launch_pass(bool apart, void (*plain)(KA...), void (*dependent)(KA..
 #define GT_HOOK(kind, begin) \
   if (hook) hook(hctx, (kind), (begin))
 
+// kept: an inverse z pass of fields that are zero outside the kept columns, which alone are
+// transformed (without `pairs`: all columns below xlim, the zero ones among them).
 template <typename R>
 static int spass(const Geom& g, void* const* fields, int nf, const void* tw, int axis, int sign,
                  cudaStream_t s, LaunchHook hook, void* hctx, int xlim = -1, int ymask = 0,
                  const int32_t* xcut0 = nullptr, int force_tx = 0, bool pairs = false, int nmem = 1,
-                 long long mstride = 0, int prefetch = 0) {
+                 long long mstride = 0, int prefetch = 0, bool kept = false) {
   const int csize = sizeof(Cplx<R>);
   const int L = axis == 1 ? g.ny : g.nz;
   const int lgL = axis == 1 ? g.lny : g.lnz;
@@ -2638,7 +2640,10 @@ static int spass(const Geom& g, void* const* fields, int nf, const void* tw, int
       dim3 grid2(ntx2, outer, nf * nmem);
       GT_HOOK(kind, true);
 #define GT_L(LG)                                                                                      \
-  if (sign > 0)                                                                                       \
+  if (sign > 0 && kept)                                                                               \
+    launch_pass(nmem == 1, k_spass2<1, LG, true, true>, k_spass2<1, LG, true, true>, grid2, c2.threads / 2, \
+                c2.smem, s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, nf, mstride);           \
+  else if (sign > 0)                                                                                  \
     launch_pass(nmem == 1, k_spass2<1, LG>, k_spass2<1, LG, true>, grid2, c2.threads / 2, c2.smem, \
                 s, f, g, tw, ls, os, c2.lgTX - 1, xlim, ymask, xcut0, nf, mstride);                    \
   else                                                                                                \
@@ -3295,7 +3300,8 @@ int launch_fft_inv(const Geom& g, const DevTables<R>& tb, void* const* spec, voi
   if ((rc = fx_spass<0>(g, spec, nf, tb.fwy, s, hook, hctx, ex, xlim, pruned ? 1 : 0, tb.xcut))) return rc;
 #else
   const bool pairs = sizeof(R) == 4;   // two columns per thread, tiles of 8 (as the pass of a step)
-  if ((rc = spass<R>(g, spec, nf, tb.twz, 2, +1, s, hook, hctx, xlim, pruned ? 3 : 0, tb.xcut, pairs ? 8 : 0, pairs)))
+  if ((rc = spass<R>(g, spec, nf, tb.twz, 2, +1, s, hook, hctx, xlim, 0, tb.xcut, pairs ? 8 : 0, pairs, 1, 0, 0,
+                     pruned != 0)))
     return rc;
   if ((rc = spass<R>(g, spec, nf, tb.twy, 1, +1, s, hook, hctx, xlim, pruned ? 1 : 0, tb.xcut, pairs ? 8 : 0, pairs)))
     return rc;

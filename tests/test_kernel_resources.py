@@ -33,3 +33,14 @@ def test_diagnostics_run_two_blocks_per_sm(unit):
     """The launch puts two blocks of 256 threads on every SM in one wave."""
     for name, (regs, _, _) in kernels(unit, "_ZN2gt6k_diagI").items():
         assert (regs + 7) // 8 * 8 * 256 * 2 <= REGISTERS, (name, regs)
+
+
+def test_inverse_y_pass_spills(lib):
+    """The step's inverse y pass is held to 64 registers for four blocks per SM; what does not
+    fit stays within 32 bytes of stores and 40 of loads, and lines of up to 64 points fit."""
+    found = {k: v for k, v in kernels("gt_kernels_f32.cu", "_ZN2gt8k_spass2ILi1E").items()
+             if re.match(r"_ZN2gt8k_spass2ILi1ELi\d+ELb[01]ELb0E", k)}
+    assert len(found) == 16   # 8 to 1024 points, launched alone or dependent
+    for name, (regs, stores, loads) in found.items():
+        short = re.match(r"_ZN2gt8k_spass2ILi1ELi[34]E", name)
+        assert regs <= 64 and stores <= (0 if short else 32) and loads <= (0 if short else 40), (name, stores, loads)
