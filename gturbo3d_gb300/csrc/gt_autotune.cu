@@ -19,7 +19,7 @@ using namespace gtc;
 // and the median kept; a candidate replaces the incumbent only if it wins by
 // more than the incumbent's own run-to-run spread (and by at least 2 %), so
 // that noise does not pick the shape.  The choice is cached per (grid,
-// precision, pruning, GPU) in a JSON-lines file.
+// precision and its passes, pruning, GPU) in a JSON-lines file.
 // ===========================================================================
 
 Tuning gtc::get_tuning(const gt_handle* h) {
@@ -48,8 +48,10 @@ std::string gtc::tuning_key(const gt_handle* h) {
   for (char& c : name)
     if (c == '"' || c == ' ') c = '_';
   char buf[256];
+  // FP64 entries name the passes they were timed with: one for passes in FP64 arithmetic ("fp64")
+  // can hold a knob that turns the fixed-point passes off (25 -> 132 ms a step at 512^3)
   std::snprintf(buf, sizeof buf, "%dx%dx%d/%s/%s/%s", h->g.nx, h->g.ny, h->g.nz,
-                h->mixed ? "mixed" : "fp64", use_pruning(h) ? "pruned" : "full", name.c_str());
+                h->mixed ? "mixed" : "fp64-fixed", use_pruning(h) ? "pruned" : "full", name.c_str());
   return buf;
 }
 
@@ -170,7 +172,15 @@ int gtc::autotune_handle(gt_handle* h, const char* cache_path, double* best_ms_o
                                    {&Tuning::fuse_stage, {0, 1}}, {&Tuning::z_split, {0, 1, 2, 3}},
                                    {&Tuning::y_prefetch, {0, 1, 2}}, {&Tuning::overlap, {0, 1}},
                                    {&Tuning::slab_pipe, {0, 1}}, {&Tuning::zf_pipe, {0, 1}}};
+  // knobs that the passes at hand do not read: FP32's y forms, and the fixed-point passes' tiles
+  auto idle = [&](int Tuning::*f) {
+    if (h->mixed) return false;
+    if (f == &Tuning::y_pairs || f == &Tuning::y_prefetch) return true;
+    return h->pm.fixed_point() && (f == &Tuning::y_tx || f == &Tuning::z_tx);
+  };
   for (const Knob& k : knobs) {
+    put_tuning(h, best);
+    if (idle(k.field)) continue;
     for (int v : k.values) {
       if (best.*(k.field) == v) continue;
       Tuning cand = best;

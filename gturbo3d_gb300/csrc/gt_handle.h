@@ -133,7 +133,7 @@ struct Tuning {
 
 Tuning get_tuning(const gt_handle* h);
 void put_tuning(gt_handle* h, const Tuning& t);
-// Cache key: grid, precision, pruning and GPU name.
+// Cache key: grid, precision and its passes, pruning and GPU name.
 std::string tuning_key(const gt_handle* h);
 // Coordinate descent over the knobs; the choice is cached in cache_path.
 int autotune_handle(gt_handle* h, const char* cache_path, double* best_ms_out);

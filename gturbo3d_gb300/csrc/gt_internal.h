@@ -163,6 +163,10 @@ struct PassTuning {
                             // points or more); 0 = one CTA per tile
   void* fx_scratch = nullptr;  // FP64: the fixed-point passes' line exponents (nullptr: FP64 arithmetic),
   long long fx_stride = 0;     // members of a batched launch this many ints apart
+  // The FP64 form's step takes the fixed-point passes: no knob selects another form of a pass.
+  bool fixed_point() const {
+    return fx_scratch && x_fused == 2 && !z_split && !overlap && !slab_pipe && !zf_pipe && !fuse_stage;
+  }
   void* stream2 = nullptr;  // the handle's second stream and the events for overlap / slab_pipe
   void* ev_fork = nullptr;
   void* ev_join = nullptr;

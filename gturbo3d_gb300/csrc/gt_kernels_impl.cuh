@@ -2698,8 +2698,7 @@ static int fx_spass(const Geom& g, void* const* fields, int nf, const void* tw, 
 // knobs that select another kernel for a pass keep FP64 arithmetic throughout
 // (nlt_phases), since the work fields' format is shared by the passes.
 static bool fx_applies(const PassTuning* pm, unsigned nm) {
-  return pm && pm->fx_scratch && (nm == 1 || pm->fx_stride > 0) && pm->x_fused == 2 && !pm->z_split &&
-         !pm->overlap && !pm->slab_pipe && !pm->zf_pipe && !pm->fuse_stage;
+  return pm && (nm == 1 || pm->fx_stride > 0) && pm->fixed_point();
 }
 
 static dim3 fx_zgrid(const Geom& g, const DevTables<double>& tb, int lgt, int pruned, unsigned nm) {
