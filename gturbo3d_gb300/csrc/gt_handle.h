@@ -69,7 +69,7 @@ struct gt_handle {
     bool broken = false;         // capture or instantiation failed once
   } sg;
   // workspace of the tangent-linear, adjoint and gradient calls, kept with the
-  // handle up to a bound (gt_tl_adj.cu)
+  // handle up to a bound (keep_limit, gt_tl_adj.cu)
   void* adj_mem = nullptr;
   size_t adj_bytes = 0;
   double* d_partials = nullptr;

@@ -33,8 +33,18 @@ struct F3 {
 // The call's workspace: one block carved into groups of three fields.  A block
 // of up to kKeep bytes stays with the handle for the next call (17 allocations and
 // frees a call before; a tangent-linear and an adjoint step at 64 x 128 x 64 mixed
-// went from 9.3 to 5.7 ms with this and the passes below).
+// went from 9.3 to 5.7 ms with this and the passes below), where a memory budget is
+// set only what it leaves beside the handle's own estimate.
 constexpr size_t kKeep = (size_t)2 << 30;
+
+size_t keep_limit(const gt_handle* h) {
+  uint64_t budget = 0;
+  size_t own = 0;
+  gt_get_memory_budget(&budget);
+  if (budget == 0) return kKeep;
+  gt_memory_estimate(&h->p, &own);
+  return budget > own ? (size_t)std::min<uint64_t>(kKeep, budget - own) : 0;
+}
 
 template <typename R>
 struct AdjWork {
@@ -47,7 +57,7 @@ struct AdjWork {
     rbytes = (size_t)h->g.nx * h->g.ny * h->g.nz * sizeof(R);
   }
   ~AdjWork() {
-    if (h->adj_bytes <= kKeep) return;
+    if (h->adj_bytes <= keep_limit(h)) return;
     cudaStreamSynchronize(h->stream);
     cudaFree(h->adj_mem);
     h->adj_mem = nullptr;
@@ -62,7 +72,11 @@ struct AdjWork {
       h->adj_mem = nullptr;
       h->adj_bytes = 0;
       const cudaError_t e = cudaMalloc(&h->adj_mem, need);
-      if (e != cudaSuccess) return cuda_fail(e, "adjoint workspace");
+      if (e != cudaSuccess) {
+        h->adj_mem = nullptr;
+        const int rc = cuda_fail(e, ("adjoint workspace of " + std::to_string(need) + " bytes").c_str());
+        return e == cudaErrorMemoryAllocation ? GT_ENOMEM : rc;
+      }
       h->adj_bytes = need;
     }
     at = static_cast<char*>(h->adj_mem);

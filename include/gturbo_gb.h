@@ -273,7 +273,12 @@ int gt_energy_noalloc(const double* bx, const double* by, const double* bz, int3
  * layout.  Adjoints are taken under <x, y> = sum over stored modes of
  * w Re(conj(x) y), w = 1 on the kx = 0 and kx = NX/2 planes and 2 elsewhere
  * (the full-spectrum inner product of real fields).  The forcing is additive
- * and state-independent, so it has no tangent. */
+ * and state-independent, so it has no tangent.
+ * These calls and gt_gradient take their workspace from the device; it stays
+ * with the handle for the next such call, up to 2 GiB and, where
+ * gt_set_memory_budget is in force, up to what that leaves beside
+ * gt_memory_estimate, and is freed by gt_destroy.  GT_ENOMEM if it cannot be
+ * had; the handle and its state are as before. */
 int gt_tl_step(gt_handle* h, const double* dbx, const double* dby, const double* dbz,
                double* ox, double* oy, double* oz);
 int gt_adj_step(gt_handle* h, const double* lx, const double* ly, const double* lz,
