@@ -271,7 +271,7 @@ void free_handle(gt_handle* h) {
   if (h->d_force) cudaFree(h->d_force);
   if (h->adj_mem) cudaFree(h->adj_mem);
   if (h->fields_mem && h->owns_fields) cudaFree(h->fields_mem);
-  if (h->stage) cudaFree(h->stage);
+  if (h->stage && h->owns_fields) cudaFree(h->stage);
   if (h->tab_mem) cudaFree(h->tab_mem);
   if (h->d_partials) cudaFree(h->d_partials);
   if (h->d_result) cudaFree(h->d_result);
@@ -576,9 +576,10 @@ int set_dev(gt_handle* h) {
 
 }  // namespace gtc
 
-// A handle; with ext_fields its twelve fields live in memory the caller
-// owns (an ensemble class slab) and are not freed with the handle.
-int gtc::create_handle(const gt_params* p, gt_handle** out, void* ext_fields) {
+// A handle; with ext_fields and ext_stage its twelve fields and its staging field
+// live in memory the caller owns (an ensemble class's slabs) and are not freed with
+// the handle.
+int gtc::create_handle(const gt_params* p, gt_handle** out, void* ext_fields, void* ext_stage) {
   if (!p || !out) return GT_EINVAL;
   *out = nullptr;
   int rc = gt_params_validate(p);
@@ -644,9 +645,11 @@ int gtc::create_handle(const gt_params* p, gt_handle** out, void* ext_fields) {
   const size_t fbytes = g.field_elems() * h->csize;
   if (ext_fields) {
     h->fields_mem = ext_fields;
+    h->stage = ext_stage;
     h->owns_fields = false;
   } else {
     CKH(cudaMalloc(&h->fields_mem, 12 * fbytes));
+    CKH(cudaMalloc(&h->stage, g.field_elems() * 16));
   }
   CKH(cudaMemsetAsync(h->fields_mem, 0, 12 * fbytes, h->stream));
   for (int c = 0; c < 3; ++c) {
@@ -654,7 +657,6 @@ int gtc::create_handle(const gt_params* p, gt_handle** out, void* ext_fields) {
     h->c[c] = dptr<void>(h->fields_mem, (3 + c) * fbytes);
   }
   for (int c = 0; c < 6; ++c) h->w[c] = dptr<void>(h->fields_mem, (6 + c) * fbytes);
-  CKH(cudaMalloc(&h->stage, g.field_elems() * 16));
   // the FP64 passes' line exponents live in the staging field, which only
   // transfers use otherwise (in stream order with the passes)
   if (!h->mixed) h->pm.fx_scratch = h->stage;
@@ -697,7 +699,7 @@ int gtc::create_handle(const gt_params* p, gt_handle** out, void* ext_fields) {
 
 extern "C" {
 
-int gt_create(const gt_params* p, gt_handle** out) { return create_handle(p, out, nullptr); }
+int gt_create(const gt_params* p, gt_handle** out) { return create_handle(p, out, nullptr, nullptr); }
 
 int gt_destroy(gt_handle* h) {
   if (!h) return GT_EINVAL;

@@ -35,7 +35,8 @@ struct EnsClass {
   std::vector<int> members;     // ensemble indices; member k's fields are slab part k
   void* slab = nullptr;         // members x 12 fields
   void* btab = nullptr;         // members' emk tables, then their (omega, dt, dt2)
-  void* fx = nullptr;           // FP64: the members' line exponents, fx_stride ints apart
+  void* stage = nullptr;        // members x staging field; FP64: from its start, while the class is
+                                // stepped, the members' line exponents, fx_stride ints apart
   int emk_len = 0;
   size_t scal_off = 0;          // byte offset of the scalars in btab
   cudaStream_t stream = nullptr;
@@ -90,7 +91,7 @@ void free_ensemble(gt_ensemble* e) {
     if (c.d_count) cudaFree(c.d_count);
     if (c.d_step) cudaFree(c.d_step);
     if (c.btab) cudaFree(c.btab);
-    if (c.fx) cudaFree(c.fx);
+    if (c.stage) cudaFree(c.stage);
     if (c.slab) cudaFree(c.slab);
     if (c.join) cudaEventDestroy(c.join);
     if (c.stream) cudaStreamDestroy(c.stream);
@@ -308,30 +309,28 @@ int gt_ensemble_create(int32_t n, const gt_params* members, gt_ensemble** out) {
     const size_t nh = (size_t)p0.nx / 2 + 1, al = 128 / esz;
     const size_t fbytes = (nh + al - 1) / al * al * p0.ny * p0.nz * esz;
     ce = cudaMalloc(&c.slab, c.members.size() * 12 * fbytes);
+    const size_t sbytes = fbytes / esz * 16;
+    if (ce == cudaSuccess) ce = cudaMalloc(&c.stage, c.members.size() * sbytes);
     if (ce != cudaSuccess) { free_ensemble(e); return ce == cudaErrorMemoryAllocation ? GT_ENOMEM : cuda_fail(ce, "slab"); }
     for (size_t k = 0; k < c.members.size(); ++k) {
       const int rc = create_handle(&members[c.members[k]], &e->m[c.members[k]],
-                                   static_cast<char*>(c.slab) + k * 12 * fbytes);
+                                   static_cast<char*>(c.slab) + k * 12 * fbytes,
+                                   static_cast<char*>(c.stage) + k * sbytes);
       if (rc) { free_ensemble(e); return rc; }
       if (e->m[c.members[k]]->g.field_elems() * esz != fbytes) { free_ensemble(e); return GT_EINVAL; }
     }
     if (p0.precision == GT_PREC_FP64) {
-      // batched fixed-point passes: the exponents of all members in one block, member 0's
-      // handle (whose knobs the class's launches use) pointing at it
+      // batched fixed-point passes: the exponents of all members side by side from the start of
+      // the staging slab, which is member 0's staging field (whose handle's knobs the class's
+      // launches use).  Transfers, and members stepped alone, use the fields one by one; both
+      // wait for the class's steps and are waited for by them.
       gt_handle* h0 = e->m[c.members[0]];
-      const size_t stride = (fx_exp_ints(h0->g.ny, h0->g.nz, h0->g.nhp) + 63) / 64 * 64;
-      ce = cudaMalloc(&c.fx, c.members.size() * stride * sizeof(int));
-      if (ce != cudaSuccess) {
-        free_ensemble(e);
-        return ce == cudaErrorMemoryAllocation ? GT_ENOMEM : cuda_fail(ce, "line exponents");
-      }
-      h0->pm.fx_scratch = c.fx;
-      h0->pm.fx_stride = (long long)stride;
+      h0->pm.fx_stride = (long long)((fx_exp_ints(h0->g.ny, h0->g.nz, h0->g.nhp) + 63) / 64 * 64);
     }
   }
   for (int i = 0; i < n; ++i) {
     if (e->m[i]) continue;
-    const int rc = create_handle(&members[i], &e->m[i], nullptr);
+    const int rc = create_handle(&members[i], &e->m[i], nullptr, nullptr);
     if (rc) { free_ensemble(e); return rc; }
   }
   ce = cudaStreamCreateWithFlags(&e->master, cudaStreamNonBlocking);

@@ -43,7 +43,7 @@ struct gt_handle {
   int csize = 16;
   cudaStream_t stream = nullptr;
   void* fields_mem = nullptr;
-  bool owns_fields = true;     // false: the fields live in an ensemble class slab
+  bool owns_fields = true;     // false: the fields and the staging field live in an ensemble class's slabs
   void* b[3]{};
   void* c[3]{};
   void* w[6]{};
@@ -123,8 +123,9 @@ int run_steps(gt_handle* h, int nsteps, const std::vector<gt::ForceEntry>& all,
 // Makes the handle's device current and clears a stale non-sticky error.
 int set_dev(gt_handle* h);
 void free_handle(gt_handle* h);
-// gt_create, with the twelve fields optionally in caller-owned device memory.
-int create_handle(const gt_params* p, gt_handle** out, void* ext_fields);
+// gt_create, with the twelve fields and the staging field optionally in
+// caller-owned device memory.
+int create_handle(const gt_params* p, gt_handle** out, void* ext_fields, void* ext_stage);
 
 // Launch-shape knobs the autotuner searches.
 struct Tuning {
