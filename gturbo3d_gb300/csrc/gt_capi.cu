@@ -481,9 +481,14 @@ bool use_step_graph(gt_handle* h, int nsteps, int pr, bool forced) {
   // kernels and their attributes outside a capture
   if (sg.steps == 0 || sg.steps + nsteps < kGraphAfter) return false;
   const int64_t before = h->launches;
-  if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
+  auto give_up = [&](cudaError_t e) {
+    g_last_error = std::string("steps launched directly, no step graph: ") + cudaGetErrorString(e);
     cudaGetLastError();
+    sg.exec = nullptr;
     sg.broken = true;
+  };
+  if (const cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed)) {
+    give_up(e);
     return false;
   }
   int rc = rk2_nlts(h, pr);
@@ -493,14 +498,12 @@ bool use_step_graph(gt_handle* h, int nsteps, int pr, bool forced) {
                   : launch_force_head<double>(g, h->b, head, h->stream, hook_fn, h);
   }
   cudaGraph_t graph = nullptr;
-  const cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
+  cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
   sg.launches = h->launches - before;
   h->launches = before;
-  if (rc || ce != cudaSuccess || cudaGraphInstantiate(&sg.exec, graph, 0) != cudaSuccess) {
-    cudaGetLastError();
-    sg.exec = nullptr;
-    sg.broken = true;
-  }
+  if (rc) ce = (cudaError_t)rc;
+  if (ce == cudaSuccess) ce = cudaGraphInstantiate(&sg.exec, graph, 0);
+  if (ce != cudaSuccess) give_up(ce);
   if (graph) cudaGraphDestroy(graph);
   return sg.exec != nullptr;
 }
@@ -554,6 +557,7 @@ int run_steps(gt_handle* h, int nsteps, const std::vector<ForceEntry>& all,
       for (; s < nsteps; ++s) {
         CK(cudaGraphLaunch(h->sg.exec, h->stream));
         h->launches += h->sg.launches;
+        ++h->sg.replays;
       }
       break;
     }
@@ -963,6 +967,7 @@ int gt_get_tuning(gt_handle* h, const char* key, int32_t* value) {
   else if (k == "z_tma") *value = h->pm.z_tma;
   else if (k == "fuse_stage") *value = h->pm.fuse_stage;
   else if (k == "z_split") *value = h->pm.z_split;
+  else if (k == "graph_replays") *value = (int32_t)std::min<int64_t>(h->sg.replays, INT32_MAX);
   else return GT_EINVAL;
   return GT_OK;
 }

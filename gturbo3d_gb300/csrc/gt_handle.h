@@ -66,7 +66,8 @@ struct gt_handle {
     std::vector<int> key;        // pruning, forcing and the launch-shape knobs it holds
     int64_t launches = 0;        // kernels a replay launches
     int64_t steps = 0;           // steps taken with this key
-    bool broken = false;         // capture or instantiation failed once
+    bool broken = false;         // capture or instantiation failed once (the reason: gt_last_error)
+    int64_t replays = 0;         // graph launches so far ("graph_replays" of gt_get_tuning)
   } sg;
   // workspace of the tangent-linear, adjoint and gradient calls, kept with the
   // handle up to a bound (keep_limit, gt_tl_adj.cu)

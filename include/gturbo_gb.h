@@ -241,7 +241,9 @@ int gt_pruning_active(gt_handle* h, int32_t* active);
  * other than the default runs the step in FP64 arithmetic. */
 int gt_set_tuning(gt_handle* h, const char* key, int32_t value);
 /* The current value of one gt_set_tuning knob (the per-grid default until
- * it is set). */
+ * it is set), or "graph_replays": the steps so far that were replayed as a graph
+ * (grids of up to 2^22 points; where a graph could not be made, steps are
+ * launched one by one and gt_last_error holds the reason). */
 int gt_get_tuning(gt_handle* h, const char* key, int32_t* value);
 
 /* Allocation-free kinetic energy, for callers that cannot allocate device
