@@ -167,7 +167,8 @@ __global__ void k_phys_cross(P3 o1, P3 o2, P3 a, P3 b, P3 c, P3 d, size_t n) {
 }
 
 // partial[block] = the block's part of sum over modes with k2 >= kmin2 of
-// fac |(curl b)|^2, products and sums in FP64; k_shell_sum adds them in order.
+// fac |(curl b)|^2: the curl in the working precision, squares and sums in FP64;
+// k_shell_sum adds the parts in order.
 constexpr int kShellThreads = 256;
 template <typename R>
 __global__ void __launch_bounds__(kShellThreads)

@@ -130,9 +130,7 @@ template <int O0, int O1, int NQ> struct FxRed {
 // Exchange scratch of TX interleaved lines (a strided tile's columns, or one x
 // line): the real parts' plane, then the imaginary parts', one padding row after
 // every 8: element e of the caller's line at (e + e / 8) TX of each plane.  Every
-// access of a stage is one base plus a compile-time offset.  Separate 8-byte
-// parts rather than 16-byte pairs: a pair's store wants four consecutive
-// registers, and the moves into them were 5 of 207 instructions a point.
+// access of a stage is one base plus a compile-time offset.
 template <int LGL, int TX> struct FxMem {
   i64* s;   // the scratch plus the line's column
   static constexpr int T = 1 << (LGL - 3);

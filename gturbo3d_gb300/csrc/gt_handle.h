@@ -113,9 +113,9 @@ int take_device_flag(gt_handle* h);
 // The truncation-aware pruned passes apply (allowed, truncating, state and
 // forcing inside the kept set).
 bool use_pruning(const gt_handle* h);
-// Host FP64 half spectrum [nz][ny][nh] <-> a device field in working precision.
 // Bytes of one host half spectrum.
 size_t spec_bytes(const gt::Geom& g);
+// Host FP64 half spectrum [nz][ny][nh] <-> a device field in working precision.
 int upload_spec(gt_handle* h, const double* host, void* dst);
 int download_spec(gt_handle* h, const void* src, double* host);
 // Enqueues nsteps RK2 steps; all[offs[s] .. offs[s+1]) are step s's forcing adds.

@@ -2686,7 +2686,7 @@ static int fx_spass(const Geom& g, void* const* fields, int nf, const void* tw, 
   const int kind = KIND == 0 || KIND == 2 ? kKYPass : kKYFwd;
   GT_HOOK(kind, true);
 #define GT_L(LG)                                                                                              \
-  launch_pass(nmem == 1, k_fx_spass<KIND, LG>, k_fx_spass<KIND, LG>, grid, kFxTileThreads, smem, \
+  launch_pass(nmem == 1, k_fx_spass<KIND, LG>, k_fx_spass<KIND, LG>, grid, kFxTileThreads, smem,              \
               s, f, g, tw, ls, os, xlim, ymask, xcut0, nf, ex, fxs, mstride);
   GT_DISPATCH_LG(lgL, GT_L)
 #undef GT_L
@@ -2726,8 +2726,8 @@ static int fx_uw(const Geom& g, const DevTables<double>& tb, void* const a[3], v
   const dim3 zigrid(zgrid.x, zgrid.y, few ? (pruned ? 6 : 6 * nm) : zgrid.z);
   GT_HOOK(kKZinvCurl, true);
 #define GT_L(LG) \
-  launch_pass(nm == 1, k_fx_zinv<LG>, k_fx_zinv<LG>, zigrid, kFxTileThreads, smem, s, pa, pw, \
-              tb, g, pruned, tb.ztl[lgt], few, ex, fxs, mstride);
+  launch_pass(nm == 1, k_fx_zinv<LG>, k_fx_zinv<LG>, zigrid, kFxTileThreads, smem, s, pa, pw, tb, g, pruned, \
+              tb.ztl[lgt], few, ex, fxs, mstride);
   GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   GT_HOOK(kKZinvCurl, false);
@@ -2759,9 +2759,8 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
     const int P = g.nx >= 256 ? 1 : 256 / g.nx;
     GT_HOOK(kKXCross, true);
 #define GT_L(LG)                                                                                        \
-  launch_pass(nm == 1, k_fx_x<LG>, k_fx_x<LG>, dim3((unsigned)(npairs / P), nm), fx_x_threads<LG>(), \
-              3 * P * strided_rows(g.nx) * 16, s, \
-      pw, g, tb.fwx, xlim, g.lnx + g.lny + g.lnz, ex, fxs, mstride);
+  launch_pass(nm == 1, k_fx_x<LG>, k_fx_x<LG>, dim3((unsigned)(npairs / P), nm), fx_x_threads<LG>(),   \
+              3 * P * strided_rows(g.nx) * 16, s, pw, g, tb.fwx, xlim, g.lnx + g.lny + g.lnz, ex, fxs, mstride);
     GT_DISPATCH_LG(g.lnx, GT_L)
 #undef GT_L
     GT_HOOK(kKXCross, false);
@@ -2775,8 +2774,8 @@ static int fx_nlt(const Geom& g, const DevTables<double>& tb, void* const a[3], 
     const dim3 ngrid = pruned ? dim3(tb.nztl[lgn], nm) : dim3((g.nh + (1 << lgn) - 1) >> lgn, g.ny, nm);
 #define GT_L(LG)                                                                                               \
   launch_pass(nm == 1, k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>,                       \
-              k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>, ngrid, kFxTileThreads / 4, 3 * zsmem / 4, s, \
-      pw, pb, po, tb, g, mode, pruned, tb.ztl[lgn], ex, fxs, bb);
+              k_fx_zfwd<(LG <= 7 ? LG : 7), fx_tile<(LG <= 7 ? LG : 7)>() / 4>, ngrid, kFxTileThreads / 4,      \
+              3 * zsmem / 4, s, pw, pb, po, tb, g, mode, pruned, tb.ztl[lgn], ex, fxs, bb);
     GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
   } else {
@@ -2889,17 +2888,14 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
       const dim3 gridf(grid.x, grid.y, fs ? (pruned ? 6 : 6 * nm) : grid.z);
 #define GT_L(LG)                                                                                    \
   launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl1<R, LG>, k_zinv_curl1<R, LG, sizeof(R) == 4>, gridf, \
-              c.threads / zcols<R>(), c.smem / 3, s, \
-              pa, pw, tb, g, c.lgTX, pruned, \
-                                                                        tb.ztl[c.lgTX], fs, mstride);
+              c.threads / zcols<R>(), c.smem / 3, s, pa, pw, tb, g, c.lgTX, pruned, tb.ztl[c.lgTX], fs, mstride);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
     } else {
 #define GT_L(LG)                                                                                   \
   launch_pass(sizeof(R) == 4 && nm == 1, k_zinv_curl<R, LG>, k_zinv_curl<R, LG, sizeof(R) == 4>, grid, \
-              c.threads / zcols<R>(), c.smem, s, \
-              pa, pw, tb, g, c.lgTX, pruned,    \
-                                                                  tb.ztl[c.lgTX], split ? 0 : 1, mstride);
+              c.threads / zcols<R>(), c.smem, s, pa, pw, tb, g, c.lgTX, pruned, tb.ztl[c.lgTX],        \
+              split ? 0 : 1, mstride);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
     }
@@ -2961,8 +2957,7 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
       if (!pm || pm->x_fused == 2) {
 #define GT_L(LG) \
   launch_pass(sizeof(R) == 4 && nm == 1, k_xbatch<R, LG>, k_xbatch<R, LG, false, sizeof(R) == 4>, \
-              dim3((unsigned)(npairs / P), nm), P * T, 3 * smem, ms, \
-              pw, gs, tb.twx, shalf, xlim, mstride);
+              dim3((unsigned)(npairs / P), nm), P * T, 3 * smem, ms, pw, gs, tb.twx, shalf, xlim, mstride);
         GT_DISPATCH_LG(gs.lnx, GT_L)
 #undef GT_L
       } else if (pm->x_fused == 3) {
@@ -3099,9 +3094,8 @@ static int nlt_phases(const Geom& g, const DevTables<R>& tb, void* const a[3], v
     } else {
 #define GT_L(LG)                                                                                   \
   launch_pass(sizeof(R) == 4 && nm == 1, k_zfwd_epi<R, LG>, k_zfwd_epi<R, LG, sizeof(R) == 4>, grid, \
-              c.threads / zfwd_cols<R>(), c.smem, s, \
-              pw, pb, po, tb, g, c.lgTX, mode, \
-                                                                 pruned, tb.ztl[c.lgTX], bb);
+              c.threads / zfwd_cols<R>(), c.smem, s, pw, pb, po, tb, g, c.lgTX, mode, pruned,           \
+              tb.ztl[c.lgTX], bb);
       GT_DISPATCH_LG(g.lnz, GT_L)
 #undef GT_L
     }
@@ -3260,10 +3254,10 @@ static int x_fields(const Geom& g, const DevTables<R>& tb, void* const* spec, vo
   const FxExp ex = fx_exp(pm->fx_scratch, g.ny, g.nz, g.nhp);
 #define GT_L(LG)                                                                                   \
   if (inverse)                                                                                     \
-    launch_pass(true, k_fx_xc2r<LG>, k_fx_xc2r<LG>, grid, threads, smem, s, ps, pr, g, \
-                tb.fwx, P, xa, ex);                                                      \
+    launch_pass(true, k_fx_xc2r<LG>, k_fx_xc2r<LG>, grid, threads, smem, s, ps, pr, g,            \
+                tb.fwx, P, xa, ex);                                                                \
   else                                                                                             \
-    launch_pass(true, k_fx_xr2c<LG>, k_fx_xr2c<LG>, grid, threads, smem, s, pr, ps, g, \
+    launch_pass(true, k_fx_xr2c<LG>, k_fx_xr2c<LG>, grid, threads, smem, s, pr, ps, g,            \
                 tb.fwx, P, g.lnx + g.lny + g.lnz, ex);
 #else
   (void)pm;
