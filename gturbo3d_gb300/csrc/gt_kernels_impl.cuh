@@ -2116,14 +2116,15 @@ k_pack_rows(double2* __restrict__ packed, Cplx<R>* __restrict__ f, size_t rows, 
 // Only modes that can be nonzero are visited (prune: the state, and with it
 // N(b), is zero outside the kept prefix of each row).  Bound by the FP64 pipe:
 // about 80 operations a mode; lanes adding to the bins one after the other took
-// 3.4 ms at 256^3 whatever the precision.  Two blocks per SM, as diag_blocks launches them:
-// left to itself the kernel takes 140-146 registers and runs in two waves of one (256^3,
-// mixed 0.426 -> 0.405 ms, FP64 0.415 -> 0.390 ms).
+// 3.4 ms at 256^3 whatever the precision.  140-146 registers admit one block per SM
+// at a time, so the launch's two per SM run in two rounds.  Held to 128 registers, with both
+// resident (mixed, with the flux, us): 256^3 492 -> 467, but 64^3 45 -> 52, 128^3 139 -> 170,
+// 256 x 64 x 128 117 -> 140, 1024 x 64 x 64 177 -> 285: rows differ in their kept lengths, and
+// the second round goes to the SMs that are done first.
 // Scalars: [0..8] glob energy terms, [9..17] enstrophy terms, [18] helicity,
 // [19] non-finite count; then E(k) [nbin], E2D(k) [nbin], flux slots [nbin].
 // ---------------------------------------------------------------------------
 constexpr int kDiagThreads = 256;
-constexpr int kDiagBlocks = 2;   // per SM
 
 // (int)sqrt(k2): a float square root decides it unless k2 is within its error
 // of a square.
@@ -2135,7 +2136,7 @@ __device__ __forceinline__ int shell_index(double k2) {
 }
 
 template <typename R>
-__global__ void __launch_bounds__(kDiagThreads, kDiagBlocks)
+__global__ void __launch_bounds__(kDiagThreads)
 k_diag(Ptr6 bb, Ptr6 nn, DevTables<R> tb, Geom g, double nu, double alpnu, double mu, double alpmu,
        int has_flux, int prune, double* partials, int nq) {
   using C = Cplx<R>;
@@ -3372,7 +3373,7 @@ int launch_point(const Geom& g, const DevTables<R>& tb, void* const a[3], int op
 int diag_blocks(const Geom& g) {
   const long long rows = (long long)g.ny * g.nz;
   long long b = (rows + 7) / 8;
-  return (int)std::min<long long>(b, 152 * kDiagBlocks);
+  return (int)std::min<long long>(b, 152 * 2);
 }
 #endif
 

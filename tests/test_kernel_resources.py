@@ -2,10 +2,6 @@
 build beside each object) against what their launches count on."""
 import re
 
-import pytest
-
-REGISTERS = 65536   # per SM
-
 
 def resources(unit):
     """{mangled kernel name: (registers, spill store bytes, spill load bytes)} of one unit."""
@@ -28,13 +24,6 @@ def kernels(unit, prefix):
     return found
 
 
-@pytest.mark.parametrize("unit", ["gt_kernels_f32.cu", "gt_kernels_f64.cu"])
-def test_diagnostics_run_two_blocks_per_sm(unit):
-    """The launch puts two blocks of 256 threads on every SM in one wave."""
-    for name, (regs, _, _) in kernels(unit, "_ZN2gt6k_diagI").items():
-        assert (regs + 7) // 8 * 8 * 256 * 2 <= REGISTERS, (name, regs)
-
-
 def test_inverse_y_pass_spills(lib):
     """The step's inverse y pass is held to 64 registers for four blocks per SM; what does not
     fit stays within 32 bytes of stores and 40 of loads, and lines of up to 64 points fit."""
@@ -42,5 +31,5 @@ def test_inverse_y_pass_spills(lib):
              if re.match(r"_ZN2gt8k_spass2ILi1ELi\d+ELb[01]ELb0E", k)}
     assert len(found) == 16   # 8 to 1024 points, launched alone or dependent
     for name, (regs, stores, loads) in found.items():
-        short = re.match(r"_ZN2gt8k_spass2ILi1ELi[34]E", name)
+        short = re.match(r"_ZN2gt8k_spass2ILi1ELi[3-6]E", name)
         assert regs <= 64 and stores <= (0 if short else 32) and loads <= (0 if short else 40), (name, stores, loads)
