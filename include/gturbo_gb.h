@@ -47,7 +47,8 @@ extern "C" {
 
 #define GT_PREC_FP64 0       /* plain form: FP64 fields and pointwise work; line
                               * transforms in 64-bit block fixed point, whose
-                              * error is below FP64 arithmetic's.  An input with
+                              * error is below FP64 arithmetic's (a run of steps,
+                              * bound by the state's own rounding, has the same).  An input with
                               * an infinity or NaN gives NaN in every value its
                               * transforms reach; inputs below 2.3e-308 count as 0 */
 #define GT_PREC_MIXED 1      /* FP32 state, FFTs and products; FP64 exponentials,
